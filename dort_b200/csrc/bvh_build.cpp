@@ -258,19 +258,15 @@ struct Collapser {
       uint32_t tri_base = uint32_t(out.tris.size());
       node.child_base = child_base;
       node.tri_base = tri_base;
-      uint32_t tri_off = 0;
       std::vector<uint32_t> leaf_tris;
+      std::vector<uint32_t> layer[2];   // the slots' first and second triangles
       for(int s = 0; s < 8; ++s) {
         int c = cand_in_slot[s];
-        if(c < 0) {
-          node.meta[s] = 0;   // an empty slot (inverted box)
-          continue;
-        }
+        if(c < 0) { continue; }   // an empty slot (inverted box)
         uint32_t b = cands[c];
         bool leaf = is_leaf(b) || bn[b].tri_total <= opts.max_leaf_tris;
         if(!leaf) {
           node.imask |= uint8_t(1u << s);
-          node.meta[s] = uint8_t(0x20 | (24 + s));
           uint32_t wi = uint32_t(out.nodes.size());
           out.nodes.emplace_back();
           queue.push_back({b, wi, cur.depth + 1});
@@ -279,30 +275,31 @@ struct Collapser {
           collect_tris(b, leaf_tris);
           uint32_t cnt = uint32_t(leaf_tris.size());
           if(cnt == 0) {
-            node.meta[s] = 0;
             for(int a = 0; a < 3; ++a) { node.qlo[a][s] = 255; node.qhi[a][s] = 0; }
             continue;
           }
-          if(cnt > 3 || tri_off + cnt > 24) {
+          if(cnt > 2) {
             err = "internal error: wide BVH leaf overflow";
             return false;
           }
-          node.meta[s] = uint8_t((((1u << cnt) - 1u) << 5) | tri_off);
-          for(uint32_t t : leaf_tris) {
-            LeafTri lt;
-            std::memset(&lt, 0, sizeof(lt));
-            const float* p0 = verts + 3 * size_t(tris[3 * size_t(t)]);
-            const float* p1 = verts + 3 * size_t(tris[3 * size_t(t) + 1]);
-            const float* p2 = verts + 3 * size_t(tris[3 * size_t(t) + 2]);
-            for(int a = 0; a < 3; ++a) {
-              lt.p0[a] = p0[a];
-              lt.e1[a] = p1[a] - p0[a];
-              lt.e2[a] = p2[a] - p0[a];
-            }
-            lt.id = t;
-            out.tris.push_back(lt);
+          node.meta[s] = uint8_t(cnt);
+          for(uint32_t k = 0; k < cnt; ++k) { layer[k].push_back(leaf_tris[k]); }
+        }
+      }
+      for(const std::vector<uint32_t>& one : layer) {
+        for(uint32_t t : one) {
+          LeafTri lt;
+          std::memset(&lt, 0, sizeof(lt));
+          const float* p0 = verts + 3 * size_t(tris[3 * size_t(t)]);
+          const float* p1 = verts + 3 * size_t(tris[3 * size_t(t) + 1]);
+          const float* p2 = verts + 3 * size_t(tris[3 * size_t(t) + 2]);
+          for(int a = 0; a < 3; ++a) {
+            lt.p0[a] = p0[a];
+            lt.e1[a] = p1[a] - p0[a];
+            lt.e2[a] = p2[a] - p0[a];
           }
-          tri_off += cnt;
+          lt.id = t;
+          out.tris.push_back(lt);
         }
       }
       out.nodes[cur.wide] = node;
@@ -322,9 +319,9 @@ struct Collapser {
 
 }  // namespace
 
-void expand_node_planes(const std::vector<WideNode>& in, std::vector<WideNodeF>& out) {
+void pack_trace_nodes(const std::vector<WideNode>& in, std::vector<TraceNode>& out) {
   out.resize(in.size());
-  for(size_t i = 0; i < in.size(); ++i) { expand_planes(in[i], out[i]); }
+  for(size_t i = 0; i < in.size(); ++i) { pack_trace_node(in[i], out[i]); }
 }
 
 bool collapse_binary_dump(const BinaryDump& tree, const float* verts, const uint32_t* tris,
@@ -361,39 +358,45 @@ bool collapse_binary_dump(const BinaryDump& tree, const float* verts, const uint
   }
   Collapser col{bn, order, verts, tris, opts, out, err};
   if(tri_count > 0 && !col.run()) { return false; }
-#ifndef DORT_NODE_QUANTIZED
-  expand_node_planes(out.nodes, out.nodes_f);
-#endif
+  pack_trace_nodes(out.nodes, out.trace);
   return true;
 }
 
-double wide_sah_cost(const WideNodeF* nodes, size_t node_count) {
+double wide_sah_cost(const TraceNode* nodes, size_t node_count) {
   if(node_count == 0) { return 0.0; }
-  auto slot_area = [](const WideNodeF& n, int s) {
-    float lo[3], hi[3];
-    for(int a = 0; a < 3; ++a) { lo[a] = n.pl[a][0][s]; hi[a] = n.pl[a][1][s]; }
-    return bw_area(lo, hi);
+  auto slot_box = [](const TraceNode& n, int s, float lo[3], float hi[3]) {
+    for(int a = 0; a < 3; ++a) {
+      auto plane = [&](int side) {
+        const uint32_t q = (n.q[a][side][s >> 2] >> (8 * (s & 3))) & 0xffu;
+        return float(double(n.p[a]) + double(q) * double(n.s[a]));
+      };
+      lo[a] = plane(0);
+      hi[a] = plane(1);
+    }
   };
+  auto tris_of = [](const TraceNode& n, int s) {
+    return ((n.masks >> (16 + s)) & 1u) + ((n.masks >> (24 + s)) & 1u);
+  };
+  float lo[3], hi[3];
   float rlo[3] = {INFINITY, INFINITY, INFINITY}, rhi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for(int s = 0; s < 8; ++s) {
-    if(nodes[0].meta[s] == 0) { continue; }
+    if(!(nodes[0].masks & (1u << s)) && !tris_of(nodes[0], s)) { continue; }
+    slot_box(nodes[0], s, lo, hi);
     for(int a = 0; a < 3; ++a) {
-      rlo[a] = std::min(rlo[a], nodes[0].pl[a][0][s]);
-      rhi[a] = std::max(rhi[a], nodes[0].pl[a][1][s]);
+      rlo[a] = std::min(rlo[a], lo[a]);
+      rhi[a] = std::max(rhi[a], hi[a]);
     }
   }
   double root = std::max(bw_area(rlo, rhi), 1e-300);
   double cost = 1.0;   // the root itself
   for(size_t i = 0; i < node_count; ++i) {
-    const WideNodeF& n = nodes[i];
+    const TraceNode& n = nodes[i];
     for(int s = 0; s < 8; ++s) {
-      if(n.meta[s] == 0) { continue; }
-      double a = slot_area(n, s) / root;
-      if(n.imask & (1u << s)) {
-        cost += a;
-      } else {
-        cost += a * double(__builtin_popcount(n.meta[s] >> 5));
-      }
+      const bool internal = n.masks & (1u << s);
+      if(!internal && !tris_of(n, s)) { continue; }
+      slot_box(n, s, lo, hi);
+      double a = bw_area(lo, hi) / root;
+      cost += internal ? a : a * double(tris_of(n, s));
     }
   }
   return cost;
@@ -426,8 +429,8 @@ bool validate_mesh(const float* verts, uint32_t vert_count, const uint32_t* tris
 bool build_wide_bvh(const float* verts, uint32_t vert_count,
                     const uint32_t* tris, uint32_t tri_count,
                     const BuildOptions& opts, WideBvh& out, std::string& err) {
-  if(opts.max_leaf_tris < 1 || opts.max_leaf_tris > 3) {
-    err = "max_leaf_tris must be 1..3";
+  if(opts.max_leaf_tris < 1 || opts.max_leaf_tris > 2) {
+    err = "max_leaf_tris must be 1..2";
     return false;
   }
   if(opts.width < 2 || opts.width > 8) {
@@ -465,9 +468,7 @@ bool build_wide_bvh(const float* verts, uint32_t vert_count,
   alloc_checkpoint();
   Collapser col{bb.nodes, bb.order_, verts, tris, opts, out, err};
   if(!col.run()) { return false; }
-#ifndef DORT_NODE_QUANTIZED
-  expand_node_planes(out.nodes, out.nodes_f);
-#endif
+  pack_trace_nodes(out.nodes, out.trace);
   return true;
 }
 

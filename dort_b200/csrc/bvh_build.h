@@ -14,14 +14,15 @@
 //     uint32_t child_base  node index of the first internal child; internal
 //                          children are contiguous, ordered by slot
 //     uint32_t tri_base    index of the node's first triangle
-//     uint8_t  meta[8]     per slot: 0 = empty; internal: 0x20 | (24 + s);
-//                          leaf: (unary triangle count << 5) | tri offset
+//     uint8_t  meta[8]     triangles of slot s when it is a leaf, else 0; a
+//                          node's triangles are its leaf slots' first ones in
+//                          slot order, then their second ones
 //     uint8_t  qlo[3][8], qhi[3][8]   quantized child boxes
 //
 // Child boxes are quantized outward with one full grid step of margin on
 // every side, so that the device slab test (rounded float arithmetic) never
-// culls a child that contains a hit.  The device traverses WideNodeF (below):
-// the same nodes with those quantized planes expanded to floats.
+// culls a child that contains a hit.  The device traverses TraceNode (below):
+// the same nodes, laid out for three 32-byte loads.
 //
 //   Triangle (48 bytes = 3 x float4, leaf order):
 //     (p0.xyz, original triangle index as bits), (e1.xyz, 0), (e2.xyz, 0)
@@ -51,21 +52,21 @@ struct alignas(16) WideNode {
 };
 static_assert(sizeof(WideNode) == 80, "WideNode must be 80 bytes");
 
-// The same node with float child planes: the quantized planes p + s q of
-// every child (margin included) rounded outward to float, so the device box
-// test needs no byte-to-float conversion.  224 bytes = 14 x uint4.
-struct alignas(16) WideNodeF {
+// The same node as the device traverses it.  96 bytes = three 32-byte loads.
+struct alignas(32) TraceNode {
+  float p[3];            // origin of the quantization grid
+  float s[3];            // its steps (powers of two)
   uint32_t child_base;
   uint32_t tri_base;
-  uint8_t meta[8];
-  uint32_t imask;
-  uint32_t pad[3];
-  float pl[3][2][8];   // [axis][0: lo, 1: hi][slot]
+  uint32_t masks;        // bits 0..7: imask; bit 16 + 8 k + s: slot s is a leaf of more than k triangles
+  uint32_t byte_one;     // 32768.f: a plane byte in its second byte makes the float 32768 + byte
+  uint32_t q[3][2][2];   // [axis][0: lo, 1: hi][slots 0..3, 4..7]: child planes, a byte per slot
+  uint32_t pad1[2];
 };
-static_assert(sizeof(WideNodeF) == 224, "WideNodeF must be 224 bytes");
+static_assert(sizeof(TraceNode) == 96, "TraceNode must be 96 bytes");
 
-// Expands quantized nodes into WideNodeF.
-void expand_node_planes(const std::vector<WideNode>& in, std::vector<WideNodeF>& out);
+// Quantized nodes as TraceNodes.
+void pack_trace_nodes(const std::vector<WideNode>& in, std::vector<TraceNode>& out);
 
 struct alignas(16) LeafTri {
   float p0[3];
@@ -83,14 +84,14 @@ constexpr double kSahTraversal = 0.5;
 
 struct BuildOptions {
   uint32_t width = 8;          // children per node, 2..8
-  uint32_t max_leaf_tris = 2;  // triangles per leaf slot, 1..3 (2: +2.7 % on the ray cast)
+  uint32_t max_leaf_tris = 2;  // triangles per leaf slot, 1..2 (2: +2.7 % on the ray cast over 3)
   uint32_t bins = 32;          // SAH bins per axis
   uint32_t threads = 0;        // 0: hardware concurrency
 };
 
 struct WideBvh {
   std::vector<WideNode> nodes;
-  std::vector<WideNodeF> nodes_f;   // float-plane nodes (traversed unless DORT_NODE_QUANTIZED)
+  std::vector<TraceNode> trace;    // the nodes as traversed
   std::vector<LeafTri> tris;
   uint32_t depth = 0;          // levels of wide nodes
   double root_lo[3] = {0, 0, 0};
@@ -98,19 +99,9 @@ struct WideBvh {
 };
 
 // The node array the device traversal reads, and its size in bytes.
-inline const void* traversal_nodes(const WideBvh& b) {
-#ifndef DORT_NODE_QUANTIZED
-  return b.nodes_f.data();
-#else
-  return b.nodes.data();
-#endif
-}
+inline const void* traversal_nodes(const WideBvh& b) { return b.trace.data(); }
 inline size_t traversal_node_bytes(const WideBvh& b) {
-#ifndef DORT_NODE_QUANTIZED
-  return b.nodes_f.size() * sizeof(WideNodeF);
-#else
-  return b.nodes.size() * sizeof(WideNode);
-#endif
+  return b.trace.size() * sizeof(TraceNode);
 }
 
 // Maximum stack depth the device traversal supports; the builder guarantees
@@ -134,10 +125,10 @@ bool collapse_binary_dump(const BinaryDump& tree, const float* verts, const uint
                           uint32_t tri_count, const BuildOptions& opts, WideBvh& out,
                           std::string& err);
 
-// Surface-area cost of a wide BVH from its float planes, relative to the
+// Surface-area cost of a wide BVH from its child planes, relative to the
 // root box: sum over visited child nodes of area, plus sum over leaf slots of
 // area x triangle count (traversal and intersection cost 1 each).
-double wide_sah_cost(const WideNodeF* nodes, size_t node_count);
+double wide_sah_cost(const TraceNode* nodes, size_t node_count);
 
 // The input checks of build_wide_bvh, with the same messages (indices in
 // range, finite coordinates of magnitude at most 1e15).

@@ -683,14 +683,13 @@ __global__ void k_plan(const DevBin* __restrict__ nodes, const uint32_t* __restr
   counts[i] = uint64_t(ci) | (uint64_t(lt) << 32);
 }
 
-template<bool kFloatPlanes>
 __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restrict__ count,
                        const uint32_t* __restrict__ leaf_idx,
                        const float* __restrict__ verts, const uint32_t* __restrict__ tris,
                        const uint32_t* __restrict__ qbin, const uint32_t* __restrict__ qwide,
                        uint32_t items, uint32_t max_leaf, const Plan* __restrict__ plans,
                        const uint64_t* __restrict__ counts, const uint64_t* __restrict__ incl,
-                       uint32_t wide_base, uint32_t tri_base0, void* __restrict__ wide_out,
+                       uint32_t wide_base, uint32_t tri_base0, TraceNode* __restrict__ wide_out,
                        LeafTri* __restrict__ leaf_out, uint32_t* __restrict__ qbin_next,
                        uint32_t* __restrict__ qwide_next, uint32_t* __restrict__ error) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -724,19 +723,23 @@ __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restr
   }
   node.child_base = child_base;
   node.tri_base = tri_base;
-  uint32_t tri_off = 0, k_internal = 0;
+  // where the next first / second triangle of a leaf slot goes
+  uint32_t tri_off[2] = {0, 0}, k_internal = 0;
   for(int s = 0; s < 8; ++s) {
     uint32_t b = p.slot_node[s];
-    if(b == ~0u) { node.meta[s] = 0; continue; }
+    if(b != ~0u && slot_is_leaf(acc, count, b, max_leaf)) { ++tri_off[1]; }
+  }
+  for(int s = 0; s < 8; ++s) {
+    uint32_t b = p.slot_node[s];
+    if(b == ~0u) { continue; }
     if(!slot_is_leaf(acc, count, b, max_leaf)) {
       node.imask |= uint8_t(1u << s);
-      node.meta[s] = uint8_t(0x20 | (24 + s));
       qbin_next[next_pos + k_internal] = b;
       qwide_next[next_pos + k_internal] = child_base + k_internal;
       ++k_internal;
       continue;
     }
-    // leaf slot: the subtree's triangles, left first (at most max_leaf <= 3)
+    // leaf slot: the subtree's triangles, left first (at most max_leaf <= 2)
     uint32_t stack[8];
     int sp = 0;
     stack[sp++] = b;
@@ -745,7 +748,7 @@ __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restr
       uint32_t x = stack[--sp];
       if(acc.leaf(x)) {
         uint32_t first = nodes[x].left & ~kLeafBit, m = nodes[x].right;
-        for(uint32_t k = 0; k < m && k < 4; ++k) {
+        for(uint32_t k = 0; k < m && k < 3; ++k) {
           uint32_t t = leaf_idx[first + k];
           LeafTri lt;
           const float* p0 = verts + 3 * size_t(tris[3 * size_t(t)]);
@@ -759,10 +762,9 @@ __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restr
           lt.id = t;
           lt.pad1 = 0.f;
           lt.pad2 = 0.f;
-          if(tri_off + cnt < tri_room) { leaf_out[tri_base + tri_off + cnt] = lt; }
+          if(cnt < 2 && tri_off[cnt] < tri_room) { leaf_out[tri_base + tri_off[cnt]++] = lt; }
           ++cnt;
         }
-        if(m > 3) { cnt = 4; }   // rejected below
       } else if(sp + 2 <= 8) {
         stack[sp++] = nodes[x].right;
         stack[sp++] = nodes[x].left;
@@ -771,21 +773,19 @@ __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restr
         return;
       }
     }
-    if(cnt == 0 || cnt > 3 || tri_off + cnt > 24 || tri_off + cnt > tri_room) {
+    if(cnt == 0 || cnt > 2) {
       atomicOr(error, 2u);
       return;
     }
-    node.meta[s] = uint8_t((((1u << cnt) - 1u) << 5) | tri_off);
-    tri_off += cnt;
+    node.meta[s] = uint8_t(cnt);
   }
-  uint32_t w = qwide[i];
-  if(kFloatPlanes) {
-    WideNodeF f;
-    expand_planes(node, f);
-    static_cast<WideNodeF*>(wide_out)[w] = f;
-  } else {
-    static_cast<WideNode*>(wide_out)[w] = node;
+  if(tri_off[1] != tri_room) {
+    atomicOr(error, 2u);
+    return;
   }
+  TraceNode packed;
+  pack_trace_node(node, packed);
+  wide_out[qwide[i]] = packed;
 }
 
 // Device buffers of one build, freed together.
@@ -1043,8 +1043,8 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
                            cudaStream_t st, DeviceBvh& out, std::string& err, BinaryDump* dump) {
   auto t0 = std::chrono::steady_clock::now();
   out = DeviceBvh();
-  if(opts.max_leaf_tris < 1 || opts.max_leaf_tris > 3) {
-    err = "max_leaf_tris must be 1..3";
+  if(opts.max_leaf_tris < 1 || opts.max_leaf_tris > 2) {
+    err = "max_leaf_tris must be 1..2";
     return false;
   }
   if(opts.width < 2 || opts.width > 8) {
@@ -1148,13 +1148,7 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
   if(!qbin || !qwide || !qbin2 || !qwide2 || !plans || !counts || !incl || !d_err) {
     return false;
   }
-#ifndef DORT_NODE_QUANTIZED
-  constexpr bool kFloat = true;
-  const size_t node_size = sizeof(WideNodeF);
-#else
-  constexpr bool kFloat = false;
-  const size_t node_size = sizeof(WideNode);
-#endif
+  const size_t node_size = sizeof(TraceNode);
   size_t wide_cap = std::max<size_t>(16, n / 4 + 16);
   void* wide = nullptr;
   if(dev_alloc(&wide, wide_cap * node_size) != cudaSuccess) {
@@ -1212,9 +1206,9 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
       wide = w2;
       wide_cap = cap2;
     }
-    k_emit<kFloat><<<blocks_for(items, 128), 128, 0, st>>>(
+    k_emit<<<blocks_for(items, 128), 128, 0, st>>>(
         nodes, count, bt.leaf_idx, verts, tris, qbin, qwide, items, opts.max_leaf_tris, plans,
-        counts, incl, wide_count, tri_count, wide, leaf, qbin2, qwide2, d_err);
+        counts, incl, wide_count, tri_count, static_cast<TraceNode*>(wide), leaf, qbin2, qwide2, d_err);
     wide_count += children;
     tri_count += leaf_tris;
     items = children;
@@ -1256,25 +1250,14 @@ extern "C" int dort_gpu_scene_bvh_cost(const dort_scene* s, double out[4]) try {
   clear_error();
   if(!s || !out) { return fail(DORT_ERR_INVALID, "null argument"); }
   size_t count = s->trace.node_count;
-  std::vector<WideNodeF> f(count);
-#ifndef DORT_NODE_QUANTIZED
+  std::vector<TraceNode> f(count);
   if(count) {
-    DG_CUDA(cudaMemcpy(f.data(), s->trace.nodes, count * sizeof(WideNodeF),
+    DG_CUDA(cudaMemcpy(f.data(), s->trace.nodes, count * sizeof(TraceNode),
                        cudaMemcpyDeviceToHost));
   }
-#else
-  std::vector<WideNode> q(count);
-  if(count) {
-    DG_CUDA(cudaMemcpy(q.data(), s->trace.nodes, count * sizeof(WideNode),
-                       cudaMemcpyDeviceToHost));
-  }
-  expand_node_planes(q, f);
-#endif
   size_t leaf_slots = 0;
-  for(const WideNodeF& n : f) {
-    for(int k = 0; k < 8; ++k) {
-      if(n.meta[k] != 0 && !(n.imask & (1u << k))) { ++leaf_slots; }
-    }
+  for(const TraceNode& n : f) {
+    for(int k = 0; k < 8; ++k) { leaf_slots += (n.masks >> (16 + k)) & 1u; }
   }
   out[0] = wide_sah_cost(f.data(), f.size());
   out[1] = double(count);
@@ -1339,15 +1322,8 @@ extern "C" int dort_gpu_check_device_bvh(const dort_scene_desc* desc, double out
   for(const LeafTri& t : dt) {
     if(t.id >= desc->tri_count || seen[t.id]++) { once = false; }
   }
-  std::vector<WideNodeF> f;
-#ifndef DORT_NODE_QUANTIZED
-  f.resize(db.node_count);
+  std::vector<TraceNode> f(db.node_count);
   if(!f.empty()) { std::memcpy(f.data(), dn.data(), dn.size()); }
-#else
-  std::vector<WideNode> q(db.node_count);
-  if(!q.empty()) { std::memcpy(q.data(), dn.data(), dn.size()); }
-  expand_node_planes(q, f);
-#endif
   out[0] = node_diff;
   out[1] = tri_diff;
   out[2] = db.node_count;

@@ -11,7 +11,7 @@
 //                     slot's octant direction from the node's centre; the
 //                     lowest score is taken first
 //   quantize_axis     8-bit conservative child planes on a power-of-two grid
-//   expand_planes     the quantized planes as floats rounded outward
+//   pack_trace_node   the quantized node in the layout the device traverses
 //
 // Every double product and sum is rounded on its own (BW_MUL / BW_ADD /
 // BW_SUB: no fused multiply-add on the device), the divisions are IEEE and
@@ -190,25 +190,30 @@ BW_HD bool quantize_node(const A& acc, const uint32_t* cands, const int cand_in_
   return true;
 }
 
-// The float-plane form of a quantized node (planes rounded outward).
-BW_HD void expand_planes(const WideNode& n, WideNodeF& f) {
-  f.child_base = n.child_base;
-  f.tri_base = n.tri_base;
-  for(int k = 0; k < 8; ++k) { f.meta[k] = n.meta[k]; }
-  f.imask = n.imask;
-  f.pad[0] = f.pad[1] = f.pad[2] = 0;
+// A quantized node in the traversal's layout.
+BW_HD void pack_trace_node(const WideNode& n, TraceNode& t) {
   for(int a = 0; a < 3; ++a) {
-    double s = ldexp(1.0, int(n.e[a]) - 127);
-    for(int k = 0; k < 8; ++k) {
-      double lo = BW_ADD(double(n.p[a]), BW_MUL(double(n.qlo[a][k]), s));
-      double hi = BW_ADD(double(n.p[a]), BW_MUL(double(n.qhi[a][k]), s));
-      float lf = float(lo), hf = float(hi);
-      if(double(lf) > lo) { lf = nextafterf(lf, -INFINITY); }
-      if(double(hf) < hi) { hf = nextafterf(hf, INFINITY); }
-      f.pl[a][0][k] = lf;
-      f.pl[a][1][k] = hf;
+    t.p[a] = n.p[a];
+    t.s[a] = float(ldexp(1.0, int(n.e[a]) - 127));
+    for(int h = 0; h < 2; ++h) {
+      uint32_t lo = 0, hi = 0;
+      for(int j = 0; j < 4; ++j) {
+        lo |= uint32_t(n.qlo[a][4 * h + j]) << (8 * j);
+        hi |= uint32_t(n.qhi[a][4 * h + j]) << (8 * j);
+      }
+      t.q[a][0][h] = lo;
+      t.q[a][1][h] = hi;
     }
   }
+  t.child_base = n.child_base;
+  t.tri_base = n.tri_base;
+  t.masks = n.imask;
+  for(int k = 0; k < 8; ++k) {
+    if(n.meta[k] > 0) { t.masks |= 1u << (16 + k); }
+    if(n.meta[k] > 1) { t.masks |= 1u << (24 + k); }
+  }
+  t.byte_one = 0x47000000u;
+  t.pad1[0] = t.pad1[1] = 0;
 }
 
 }  // namespace dort_gpu

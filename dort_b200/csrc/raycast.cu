@@ -1,61 +1,61 @@
 // Ray-cast kernels and their C-ABI entry points.
 //
-// One thread per ray inside a persistent grid (one wave of resident blocks);
-// each warp takes 32 consecutive rays at a time from a device work counter,
-// so warps whose rays finish early pick up new ones instead of idling until
-// the slowest ray of a static block is done.  Rays are read as two 16-byte
-// loads, results written as one u32 + three floats per ray.
+// A persistent grid (one wave of resident blocks) traces the rays as one queue
+// (trace_queue.cuh).  Rays are read as two 16-byte loads, results written as
+// one u32 + three floats per ray.
 #include <cstring>
 #include <string>
 
 #include "common.h"
-#include "trace.cuh"
+#include "trace_queue.cuh"
 
 namespace dort_gpu {
 
 constexpr int kRaycastBlock = 128;
-// The work counter runs past ray_count by at most one fetch per warp; entries
+// The work counter runs past ray_count by at most 64 entries per warp; entries
 // are limited so that it cannot wrap.
 constexpr size_t kRaycastMaxRays = 0xff000000u;
 
-// Launch bound without a minimum block count (DORT_RAYCAST_MIN_BLOCKS
-// unset): the compiler then keeps the kernel at 60-64 registers, 2,476
-// Mrays/s on the ray-cast workload.  An explicit minimum of 1 raised it to 96
-// registers (2,044 Mrays/s); minimums of 9, 10, 12 and 16 measured 2,384,
-// 2,001, 1,309 and 692 Mrays/s.
-#ifdef DORT_RAYCAST_MIN_BLOCKS
-#define DORT_RAYCAST_BOUNDS __launch_bounds__(kRaycastBlock, DORT_RAYCAST_MIN_BLOCKS)
-#else
-#define DORT_RAYCAST_BOUNDS __launch_bounds__(kRaycastBlock)
-#endif
+// The ray-cast queue of trace_queue: rays in, hits out.
+template<bool ANY_HIT>
+struct RaycastQueue {
+  const TraceScene& sc;
+  const float4* __restrict__ rays;
+  uint32_t* __restrict__ out_prim;
+  float* __restrict__ out_tb;
+  __device__ __forceinline__ const TraceScene& scene() const { return sc; }
+  __device__ __forceinline__ void load(uint32_t i, TravState& s) const {
+    float4 r0 = __ldcs(rays + 2 * size_t(i));
+    float4 r1 = __ldcs(rays + 2 * size_t(i) + 1);
+    trav_init(s, sc, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w);
+  }
+  __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) const {
+    if(!mine) { return; }
+    if(ANY_HIT) {
+      out_prim[i] = s.best.prim != kMiss ? 1u : 0u;
+      return;
+    }
+    out_prim[i] = s.best.prim;
+    if(s.best.prim != kMiss) {
+      out_tb[3 * size_t(i)] = s.best.t;
+      out_tb[3 * size_t(i) + 1] = s.best.b1;
+      out_tb[3 * size_t(i) + 2] = s.best.b2;
+    }
+  }
+};
+
+// 64 registers (8 resident blocks): 9 and 10 blocks measured 2 and 9 % slower
+// on incoherent rays (spills), 6 and 7 no faster.  What bounds it on the
+// 1M-triangle soup (4M rays): camera rays, instruction issue (81 % of the
+// active cycles); bounce rays, the L1 data pipe (76 %) and issue (74 %)
+// together.
 template<bool ANY_HIT, int WT = kTriMt>
-__global__ void DORT_RAYCAST_BOUNDS
+__global__ void __launch_bounds__(kRaycastBlock, 8)
 raycast_kernel(TraceScene sc, const float4* __restrict__ rays, uint32_t ray_count,
                uint32_t* __restrict__ out_prim, float* __restrict__ out_tb,
                uint32_t* __restrict__ work) {
-  const uint32_t lane = threadIdx.x & 31u;
-  for(;;) {
-    uint32_t base = 0;
-    if(lane == 0) { base = atomicAdd(work, 32u); }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if(base >= ray_count) { break; }
-    uint32_t i = base + lane;
-    if(i < ray_count) {
-      float4 r0 = __ldcs(rays + 2 * size_t(i));
-      float4 r1 = __ldcs(rays + 2 * size_t(i) + 1);
-      Hit h = trace_ray<ANY_HIT, true, WT>(sc, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w);
-      if(ANY_HIT) {
-        out_prim[i] = h.prim != kMiss ? 1u : 0u;
-      } else {
-        out_prim[i] = h.prim;
-        if(h.prim != kMiss) {
-          out_tb[3 * size_t(i)] = h.t;
-          out_tb[3 * size_t(i) + 1] = h.b1;
-          out_tb[3 * size_t(i) + 2] = h.b2;
-        }
-      }
-    }
-  }
+  RaycastQueue<ANY_HIT> q{sc, rays, out_prim, out_tb};
+  trace_queue<ANY_HIT, true, WT>(q, ray_count, work);
 }
 
 static int persistent_blocks(const void* kernel, int block) {

@@ -6,12 +6,12 @@
 // and the triangle tests TriangleUv::hit / Triangle::hit_p
 // (triangle.cpp:14-46, 102-134).
 //
-// Traversal: node groups (base index, 8 child-hit bits << 24 | internal-slot
-// mask) on a per-thread stack; child slots are visited in an order fixed by
+// Traversal: node groups (base index, internal-slot mask << 8 | child-hit
+// bits) on a per-thread stack; child slots are visited in an order fixed by
 // the ray octant (slot bit index XOR octant), so no per-node sort is needed.
-// Child boxes are tested with fused multiply-adds on the planes (rounded
-// outward) and a relative widening that covers the rounding of that
-// arithmetic (DG_BOX_HIT); together with the one-step quantization margin the
+// Child boxes are tested with fused multiply-adds on the quantized planes and
+// a relative widening that covers the rounding of that arithmetic
+// (DORT_SLAB_FAR_WIDEN); together with the one-step quantization margin the
 // test never culls a box containing a hit.
 //
 // Triangle test: the reference's Moller-Trumbore operations in the
@@ -32,14 +32,10 @@
 #define DG_ADD(a, b) __fadd_rn(a, b)
 #define DG_SUB(a, b) __fsub_rn(a, b)
 #define DG_RCP(a) __frcp_rn(a)
-#define DG_U2F(u) __uint2float_rn(u)
-#define DG_CLZ(x) __clz(x)
 #define DG_POPC(x) __popc(x)
-#define DG_FFS(x) __ffs(x)
 #define DG_LDG(p) __ldg(p)
 #define DG_AS_FLOAT(u) __uint_as_float(u)
 #define DG_AS_UINT(f) __float_as_uint(f)
-#define DG_BYTE_F(w, j) __uint2float_rn(((w) >> (8 * (j))) & 0xffu)
 #define DG_FMA(a, b, c) fmaf(a, b, c)
 #define DG_RCP_FAST(a) __frcp_rn(a)
 // three-input float max / min (one instruction on sm_100a; exact, like two
@@ -54,8 +50,26 @@ __device__ __forceinline__ float dg_min3(float a, float b, float c) {
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// reciprocal to one unit in the last place (the box test's, see
+// DORT_SLAB_FAR_WIDEN)
+__device__ __forceinline__ float dg_rcp_approx(float a) {
+  float d;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(d) : "f"(a));
+  return d;
+}
+#define DG_RCP_APPROX(a) dg_rcp_approx(a)
 #define DG_MAX3(a, b, c) dg_max3(a, b, c)
 #define DG_MIN3(a, b, c) dg_min3(a, b, c)
+// the sign bit of `f` shifted into the low end of `m` (one funnel shift)
+#define DG_PUSH_SIGN(m, f) __funnelshift_l(__float_as_uint(f), m, 1)
+// byte j of `w` as the float 32768 + byte, `one` = the bits of 32768.f: one
+// byte permutation.  (`one` comes from the node: as a constant the compiler
+// moves it into a register before every one of a node's 48 permutations.)
+#define DG_BYTE_FLOAT(w, one, j) \
+  __uint_as_float(__byte_perm(w, one, 0x7404u | (uint32_t(j) << 4)))
+// byte j of `w` as the float 65536 + byte: one dot product of bytes (128 steps
+// of 2^-7 added to the bits of 65536.f), on another pipe than the permutations
+#define DG_BYTE_FLOAT_DP(w, j) __uint_as_float(__dp4a(w, 0x80u << (8 * (j)), 0x47800000u))
 #else
 namespace dort_gpu {
 inline float host_as_float(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
@@ -65,18 +79,18 @@ inline uint32_t host_as_uint(float f) { uint32_t u; std::memcpy(&u, &f, 4); retu
 #define DG_ADD(a, b) ((a) + (b))
 #define DG_SUB(a, b) ((a) - (b))
 #define DG_RCP(a) (1.f / (a))
-#define DG_U2F(u) (float(u))
-#define DG_CLZ(x) __builtin_clz(x)
 #define DG_POPC(x) __builtin_popcount(x)
-#define DG_FFS(x) __builtin_ffs(int(x))
 #define DG_LDG(p) (*(p))
 #define DG_AS_FLOAT(u) ::dort_gpu::host_as_float(u)
 #define DG_AS_UINT(f) ::dort_gpu::host_as_uint(f)
-#define DG_BYTE_F(w, j) (float(((w) >> (8 * (j))) & 0xffu))
 #define DG_FMA(a, b, c) std::fma(a, b, c)
 #define DG_RCP_FAST(a) (1.f / (a))
+#define DG_RCP_APPROX(a) (1.f / (a))
 #define DG_MAX3(a, b, c) fmaxf(fmaxf(a, b), c)
 #define DG_MIN3(a, b, c) fminf(fminf(a, b), c)
+#define DG_PUSH_SIGN(m, f) (((m) << 1) | (DG_AS_UINT(f) >> 31))
+#define DG_BYTE_FLOAT(w, one, j) (32768.f + float(((w) >> (8 * (j))) & 0xffu))
+#define DG_BYTE_FLOAT_DP(w, j) (65536.f + float(((w) >> (8 * (j))) & 0xffu))
 #endif
 #define DG_HD __host__ __device__ __forceinline__
 
@@ -225,10 +239,6 @@ DG_HD bool wt_hit(const WtRay& r, float4 p0, float4 p1, float4 p2, float ox, flo
   return true;
 }
 
-DG_HD float byte_to_float(uint32_t w, int j) {
-  return DG_BYTE_F(w, j);
-}
-
 // Widening of the slab test.  The plane distances t carry a relative
 // rounding error below 2^-20 of |t| (> 8 ulp).  Widening both ends by that,
 // tnear - |tnear| 2^-20 <= tfar + |tfar| 2^-20, takes two fused multiply-adds
@@ -239,124 +249,81 @@ DG_HD float byte_to_float(uint32_t w, int j) {
 // 2^-18); with both < 0, |tfar| > |tnear| and 2^-18 |tfar| exceeds the two
 // margins together; with tnear >= 0 > tfar both forms reject).
 #define DORT_SLAB_FAR_WIDEN 3.814697265625e-6f
-#define DG_BOX_HIT(tn, tf) ((tn) <= DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, (tf)))
 
-// Tests the 8 child boxes of one node; returns the hit mask: bits 24..31 =
-// internal children (bit 24 + (slot ^ oct_inv)), bits 0..23 = triangles
-// relative to the node's tri_base.
-DG_HD uint32_t node_hitmask(
-    const uint4& n0, const uint4& n1, const uint4& n2, const uint4& n3, const uint4& n4,
-    float ox, float oy, float oz, float ix, float iy, float iz,
-    float t_min, float t_max, uint32_t oct_inv4) {
-  float px = DG_AS_FLOAT(n0.x), py = DG_AS_FLOAT(n0.y), pz = DG_AS_FLOAT(n0.z);
-  float sx = DG_AS_FLOAT((n0.w & 0xffu) << 23);
-  float sy = DG_AS_FLOAT(((n0.w >> 8) & 0xffu) << 23);
-  float sz = DG_AS_FLOAT(((n0.w >> 16) & 0xffu) << 23);
-  float adj_ix = sx * ix, adj_iy = sy * iy, adj_iz = sz * iz;
-  float adj_ox = (px - ox) * ix, adj_oy = (py - oy) * iy, adj_oz = (pz - oz) * iz;
+// 32 bytes of a node with one load (32-byte aligned).
+DG_HD void load_32(const uint4* p, uint32_t v[8]) {
+#ifdef __CUDA_ARCH__
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7])
+      : "l"(p));
+#else
+  std::memcpy(v, p, 32);
+#endif
+}
 
+constexpr uint32_t kNodeWords = 6;   // uint4 words per TraceNode
+
+// Tests the 8 child boxes of one node (TraceNode, as three 32-byte loads):
+// bit s of the result is set when the ray's [t_min, t_max] meets slot s's
+// box (t_far_max = t_max widened).  Empty slots have no bit in either mask of
+// the node, so their result does not matter.
+//
+// What bounds it: a node of 8 byte-quantized boxes fetched as three 32-byte
+// loads costs the L1 data pipe a third of the same node with float planes in
+// fourteen 16-byte loads (a warp of 13 divergent lanes: 40 against 123 cycles
+// per node step on one SM; the pipe was 82 % busy), and then the instructions
+// count: half-rate integer and min / max operations (the ALU pipe) first.
+// Hence one operation per plane byte, near planes on the ALU pipe and far
+// planes on the FMA pipe (all 48 on the ALU pipe: +2 % on the camera rays),
+// and one funnel shift per child to collect the results as sign bits.
+DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
+                         float ox, float oy, float oz, float ix, float iy, float iz,
+                         float t_min, float t_far_max) {
+  // t of plane q on an axis: (p + s q - o) i = (32768 + q) a + b = (65536 + q) a + c
+  // (b and c are off by less than a / 128, of the margin's a)
+  const float ax = DG_AS_FLOAT(n0[3]) * ix, ay = DG_AS_FLOAT(n0[4]) * iy,
+              az = DG_AS_FLOAT(n0[5]) * iz;
+  const float bx = DG_FMA(-32768.f, ax, (DG_AS_FLOAT(n0[0]) - ox) * ix);
+  const float by = DG_FMA(-32768.f, ay, (DG_AS_FLOAT(n0[1]) - oy) * iy);
+  const float bz = DG_FMA(-32768.f, az, (DG_AS_FLOAT(n0[2]) - oz) * iz);
+  const float cx = DG_FMA(-32768.f, ax, bx), cy = DG_FMA(-32768.f, ay, by),
+              cz = DG_FMA(-32768.f, az, bz);
   // near / far plane bytes per axis, by direction sign
   const bool nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
-  uint32_t near_x[2] = { nx ? n3.z : n2.x, nx ? n3.w : n2.y };
-  uint32_t far_x[2]  = { nx ? n2.x : n3.z, nx ? n2.y : n3.w };
-  uint32_t near_y[2] = { ny ? n4.x : n2.z, ny ? n4.y : n2.w };
-  uint32_t far_y[2]  = { ny ? n2.z : n4.x, ny ? n2.w : n4.y };
-  uint32_t near_z[2] = { nz ? n4.z : n3.x, nz ? n4.w : n3.y };
-  uint32_t far_z[2]  = { nz ? n3.x : n4.z, nz ? n3.y : n4.w };
-
-  uint32_t hitmask = 0;
+  const uint32_t near_x[2] = { nx ? n1[4] : n1[2], nx ? n1[5] : n1[3] };
+  const uint32_t far_x[2]  = { nx ? n1[2] : n1[4], nx ? n1[3] : n1[5] };
+  const uint32_t near_y[2] = { ny ? n2[0] : n1[6], ny ? n2[1] : n1[7] };
+  const uint32_t far_y[2]  = { ny ? n1[6] : n2[0], ny ? n1[7] : n2[1] };
+  const uint32_t near_z[2] = { nz ? n2[4] : n2[2], nz ? n2[5] : n2[3] };
+  const uint32_t far_z[2]  = { nz ? n2[2] : n2[4], nz ? n2[3] : n2[5] };
+  const uint32_t one = n1[1];
+  uint32_t miss = 0;
 #pragma unroll
-  for(int h = 0; h < 2; ++h) {
-    uint32_t meta4 = h ? n1.w : n1.z;
-    uint32_t is_inner4 = (meta4 & (meta4 << 1)) & 0x10101010u;
-    uint32_t inner_mask4 = (is_inner4 >> 4) * 0xffu;
-    uint32_t bit_index4 = (meta4 ^ (oct_inv4 & inner_mask4)) & 0x1f1f1f1fu;
-    uint32_t child_bits4 = (meta4 >> 5) & 0x07070707u;
-#pragma unroll
-    for(int j = 0; j < 4; ++j) {
-      float tnx = fmaf(byte_to_float(near_x[h], j), adj_ix, adj_ox);
-      float tny = fmaf(byte_to_float(near_y[h], j), adj_iy, adj_oy);
-      float tnz = fmaf(byte_to_float(near_z[h], j), adj_iz, adj_oz);
-      float tfx = fmaf(byte_to_float(far_x[h], j), adj_ix, adj_ox);
-      float tfy = fmaf(byte_to_float(far_y[h], j), adj_iy, adj_oy);
-      float tfz = fmaf(byte_to_float(far_z[h], j), adj_iz, adj_oz);
-      float tnear = DG_MAX3(tnx, tny, fmaxf(tnz, t_min));
-      float tfar = DG_MIN3(tfx, tfy, fminf(tfz, t_max));
-      bool hit = DG_BOX_HIT(tnear, tfar);
-      if(hit) {
-        uint32_t bits = (child_bits4 >> (8 * j)) & 0xffu;
-        uint32_t bidx = (bit_index4 >> (8 * j)) & 0xffu;
-        hitmask |= bits << bidx;
-      }
-    }
+  for(int s = 7; s >= 0; --s) {
+    const int h = s >> 2, j = s & 3;
+    const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(near_x[h], one, j), ax, bx),
+                             DG_FMA(DG_BYTE_FLOAT(near_y[h], one, j), ay, by),
+                             DG_FMA(DG_BYTE_FLOAT(near_z[h], one, j), az, bz));
+    float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT_DP(far_x[h], j), ax, cx),
+                       DG_FMA(DG_BYTE_FLOAT_DP(far_y[h], j), ay, cy),
+                       DG_FMA(DG_BYTE_FLOAT_DP(far_z[h], j), az, cz));
+    tf = DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, tf);
+    // tn <= tf, t_min <= tf and tn <= t_far_max: no difference is negative
+    miss = DG_PUSH_SIGN(miss, DG_MIN3(tf - tn, tf - t_min, t_far_max - tn));
   }
-  return hitmask;
+  return ~miss & 0xffu;
 }
 
-// Node words per node in device memory: the 224-byte node with float planes
-// (bvh_build.h WideNodeF), or in builds with DORT_NODE_QUANTIZED the 80-byte
-// quantized node.  The float planes cost 2.8x the node bytes but no
-// byte-to-float conversions (48 per node) in the box test, which is issue
-// bound: +7 % rays/s on the ray-cast and wavefront workloads.
-#ifndef DORT_NODE_QUANTIZED
-constexpr uint32_t kNodeWords = 14;
-#else
-constexpr uint32_t kNodeWords = 5;
-#endif
-
-// Child test of a float-plane node (WideNodeF): the same hit mask as
-// node_hitmask.  nox = -ox * ix (per ray), so each plane costs one FMA.
-DG_HD uint32_t node_hitmask_f(const uint4* np, uint4 h0, float ix, float iy, float iz,
-                              float nox, float noy, float noz, float t_min, float t_max,
-                              uint32_t oct_inv4) {
-  const float4* pl = reinterpret_cast<const float4*>(np + 2);   // [axis][lo, hi][8]
-  const int sx = ix < 0.f ? 2 : 0, sy = iy < 0.f ? 2 : 0, sz = iz < 0.f ? 2 : 0;
-  uint32_t hitmask = 0;
-#pragma unroll
-  for(int h = 0; h < 2; ++h) {
-    float4 nx = DG_LDG(pl + sx + h), fx = DG_LDG(pl + (2 - sx) + h);
-    float4 ny = DG_LDG(pl + 4 + sy + h), fy = DG_LDG(pl + 4 + (2 - sy) + h);
-    float4 nz = DG_LDG(pl + 8 + sz + h), fz = DG_LDG(pl + 8 + (2 - sz) + h);
-    uint32_t meta4 = h ? h0.w : h0.z;
-    uint32_t is_inner4 = (meta4 & (meta4 << 1)) & 0x10101010u;
-    uint32_t inner_mask4 = (is_inner4 >> 4) * 0xffu;
-    uint32_t bit_index4 = (meta4 ^ (oct_inv4 & inner_mask4)) & 0x1f1f1f1fu;
-    uint32_t child_bits4 = (meta4 >> 5) & 0x07070707u;
-    const float nxa[4] = {nx.x, nx.y, nx.z, nx.w}, fxa[4] = {fx.x, fx.y, fx.z, fx.w};
-    const float nya[4] = {ny.x, ny.y, ny.z, ny.w}, fya[4] = {fy.x, fy.y, fy.z, fy.w};
-    const float nza[4] = {nz.x, nz.y, nz.z, nz.w}, fza[4] = {fz.x, fz.y, fz.z, fz.w};
-#pragma unroll
-    for(int j = 0; j < 4; ++j) {
-      float tnear = DG_MAX3(fmaf(nxa[j], ix, nox), fmaf(nya[j], iy, noy),
-                            fmaxf(fmaf(nza[j], iz, noz), t_min));
-      float tfar = DG_MIN3(fmaf(fxa[j], ix, nox), fmaf(fya[j], iy, noy),
-                           fminf(fmaf(fza[j], iz, noz), t_max));
-      bool hit = DG_BOX_HIT(tnear, tfar);
-      if(hit) {
-        uint32_t bits = (child_bits4 >> (8 * j)) & 0xffu;
-        uint32_t bidx = (bit_index4 >> (8 * j)) & 0xffu;
-        hitmask |= bits << bidx;
-      }
-    }
-  }
-  return hitmask;
-}
-
-// Traversal state of one ray.  trav_step advances it by one node (the
-// node's child boxes, then the triangles of its leaf children); trace_ray
-// runs the steps of one ray to the end.  (Handing a finished lane a new ray
-// between steps, with a warp vote per step, measured slower than running
-// each warp's 32 rays to the end: 1,882 against 2,460 Mrays/s on the ray
-// cast at the best threshold, and a slower extension stage at every one.)
+// Traversal state of one ray.  trav_node visits one node, trav_tri tests one
+// triangle, trav_step does a node and its triangles; trace_ray runs the steps
+// of one ray to the end, trace_queue (trace_queue.cuh) those of a whole queue.
 struct TravState {
   float ox, oy, oz, dx, dy, dz, t_min;
   float ix, iy, iz;
-#ifndef DORT_NODE_QUANTIZED
-  float nox, noy, noz;   // -o * inv: one FMA per plane
-#endif
-  uint32_t oct_inv, oct_inv4;
+  uint32_t near4, near2, near1;   // slots on the ray's near side, by slot bit 2, 1, 0
   WtRay wt;              // the watertight test's ray frame (WT traversals)
-  uint2 group;           // current node group: (base, child-hit bits << 24 | internal mask)
+  uint2 group;           // current node group: (base, internal mask << 8 | child-hit bits)
   int sp;                // entries on the caller's stack
   Hit best;              // closest hit so far (best.t = t_max while none)
 };
@@ -370,21 +337,17 @@ DG_HD void trav_init(TravState& s, const TraceScene& sc, float ox, float oy, flo
   s.best.prim = kMiss;
   // Box-test reciprocals; zero components become tiny so no NaN appears.
   const float tiny = 1e-20f;
-  s.ix = 1.f / (fabsf(dx) < tiny ? copysignf(tiny, dx) : dx);
-  s.iy = 1.f / (fabsf(dy) < tiny ? copysignf(tiny, dy) : dy);
-  s.iz = 1.f / (fabsf(dz) < tiny ? copysignf(tiny, dz) : dz);
-  s.oct_inv = (s.ix < 0.f ? 0u : 1u) | (s.iy < 0.f ? 0u : 2u) | (s.iz < 0.f ? 0u : 4u);
-  s.oct_inv4 = s.oct_inv * 0x01010101u;
-#ifndef DORT_NODE_QUANTIZED
-  s.nox = -ox * s.ix;
-  s.noy = -oy * s.iy;
-  s.noz = -oz * s.iz;
-#endif
+  s.ix = DG_RCP_APPROX(fabsf(dx) < tiny ? copysignf(tiny, dx) : dx);
+  s.iy = DG_RCP_APPROX(fabsf(dy) < tiny ? copysignf(tiny, dy) : dy);
+  s.iz = DG_RCP_APPROX(fabsf(dz) < tiny ? copysignf(tiny, dz) : dz);
+  s.near4 = s.iz < 0.f ? 0xf0u : 0x0fu;
+  s.near2 = s.iy < 0.f ? 0xccu : 0x33u;
+  s.near1 = s.ix < 0.f ? 0xaau : 0x55u;
   s.wt = wt_setup(dx, dy, dz);
   s.sp = 0;
-  // root group: internal bit 31 with an empty internal-slot mask -> node 0;
-  // an empty tree starts finished
-  s.group = make_uint2(0u, sc.node_count ? 0x80000000u : 0u);
+  // root group: one child with an empty internal-slot mask -> node 0; an
+  // empty tree starts finished
+  s.group = make_uint2(0u, sc.node_count ? 1u : 0u);
 }
 
 // Traversal stacks.  A node group is pushed per level descended, so a ray's
@@ -448,71 +411,89 @@ using TraceStack = LocalStack;
 // (TraceScene::watertight).
 enum : int { kTriMt = 0, kTriWatertight = 1, kTriByScene = 2 };
 
-// One traversal step; returns true when the ray is finished (s.best holds
-// the closest hit, or for ANY_HIT the first hit found, or prim = kMiss).
-template<bool ANY_HIT, bool EXACT_MT, class Stack, int WT = kTriMt>
-DG_HD bool trav_step(TravState& s, const TraceScene& sc, Stack& stack) {
-  if((s.group.y & 0xff000000u) == 0u) {
-    if(s.sp == 0) { return true; }
-    s.group = stack.pop(--s.sp);
-  }
-  uint32_t bit = 31u - DG_CLZ(s.group.y & 0xff000000u);
-  s.group.y &= ~(1u << bit);
-  uint32_t slot = (bit - 24u) ^ s.oct_inv;
-  uint32_t node_idx = s.group.x + DG_POPC(s.group.y & 0xffu & ((1u << slot) - 1u));
+// A node's leaf triangles that a ray still has to test: x = index of the
+// node's first triangle, y = their bits (low half, bit 8 k + s: triangle k of
+// slot s) under the bits of all its triangles (high half).
+DG_HD bool leaf_empty(uint2 leaf) { return (leaf.y & 0xffffu) == 0u; }
+
+// Whether the ray has nodes left (the current group is refilled from the
+// stack as soon as it is empty).
+DG_HD bool group_left(const TravState& s) { return (s.group.y & 0xffu) != 0u; }
+
+// Visits the next node (there must be one, group_left): its hit children
+// become the current group, its hit leaf slots are returned.
+template<class Stack>
+DG_HD uint2 trav_node(TravState& s, const TraceScene& sc, Stack& stack) {
+  // the hit child nearest in octant order: prefer the near half by slot bit
+  // 2, then bit 1, then bit 0
+  uint32_t pick = s.group.y & 0xffu;
+  pick = (pick & s.near4) ? pick & s.near4 : pick;
+  pick = (pick & s.near2) ? pick & s.near2 : pick;
+  pick = (pick & s.near1) ? pick & s.near1 : pick;
+  s.group.y ^= pick;
+  uint32_t node_idx = s.group.x + DG_POPC((s.group.y >> 8) & (pick - 1u));
 
   const uint4* np = sc.nodes + kNodeWords * size_t(node_idx);
-#ifndef DORT_NODE_QUANTIZED
-  uint4 h0 = DG_LDG(np);
-  uint32_t imask = DG_LDG(&np[1].x);
-  uint32_t hitmask = node_hitmask_f(np, h0, s.ix, s.iy, s.iz, s.nox, s.noy, s.noz, s.t_min,
-                                    s.best.t, s.oct_inv4);
-  const uint32_t child_base = h0.x, tri_base = h0.y;
-#else
-  uint4 n0 = DG_LDG(np), n1 = DG_LDG(np + 1), n2 = DG_LDG(np + 2);
-  uint4 n3 = DG_LDG(np + 3), n4 = DG_LDG(np + 4);
-  uint32_t hitmask = node_hitmask(n0, n1, n2, n3, n4, s.ox, s.oy, s.oz, s.ix, s.iy, s.iz,
-                                  s.t_min, s.best.t, s.oct_inv4);
-  const uint32_t child_base = n1.x, tri_base = n1.y, imask = n0.w >> 24;
-#endif
+  uint32_t n0[8], n1[8], n2[8];
+  load_32(np, n0);
+  load_32(np + 2, n1);
+  load_32(np + 4, n2);
+  const uint32_t hits = node_hits(n0, n1, n2, s.ox, s.oy, s.oz, s.ix, s.iy, s.iz, s.t_min,
+                                  DG_FMA(fabsf(s.best.t), DORT_SLAB_FAR_WIDEN, s.best.t));
+  const uint32_t child_base = n0[6], tri_base = n0[7], masks = n1[0];
 
-  uint32_t child_hits = hitmask & 0xff000000u;
-  if(child_hits) {
-    if(s.group.y & 0xff000000u) {
+  const uint32_t inner = hits & masks & 0xffu;
+  if(inner) {
+    if(group_left(s)) {
       // sp < kTraceStack: each push descends one level and the builder
       // bounds the depth by kMaxWideDepth.
       stack.push(s.sp++, s.group);
     }
-    s.group = make_uint2(child_base, child_hits | imask);
+    s.group = make_uint2(child_base, (masks << 8) | inner);
+  } else if(!group_left(s) && s.sp > 0) {
+    s.group = stack.pop(--s.sp);
   }
+  return make_uint2(tri_base, (masks & 0xffff0000u) | ((hits * 0x101u) & (masks >> 16)));
+}
 
-  uint32_t tri_hits = hitmask & 0x00ffffffu;
-  while(tri_hits) {
-    uint32_t b = DG_FFS(tri_hits) - 1u;
-    tri_hits &= tri_hits - 1u;
-    const float4* tp = sc.tris + 3 * size_t(tri_base + b);
-    float4 a = DG_LDG(tp), e1 = DG_LDG(tp + 1), e2 = DG_LDG(tp + 2);
-    float t, b1, b2;
-    bool h;
-    if(WT == kTriWatertight || (WT == kTriByScene && sc.watertight)) {
-      h = wt_hit(s.wt, a, e1, e2, s.ox, s.oy, s.oz, s.t_min, s.best.t, t, b1, b2);
-    } else {
-      h = EXACT_MT
-          ? mt_exact(a, e1, e2, s.ox, s.oy, s.oz, s.dx, s.dy, s.dz, s.t_min, s.best.t, t, b1, b2)
-          : mt_fast(a, e1, e2, s.ox, s.oy, s.oz, s.dx, s.dy, s.dz, s.t_min, s.best.t, t, b1, b2);
-    }
-    if(h) {
-      uint32_t id = DG_AS_UINT(a.w);
-      if(ANY_HIT) {
-        s.best.t = t; s.best.b1 = b1; s.best.b2 = b2; s.best.prim = id;
-        return true;
-      }
-      if(s.best.prim == kMiss || t < s.best.t || id > s.best.prim) {
-        s.best.t = t; s.best.b1 = b1; s.best.b2 = b2; s.best.prim = id;
-      }
+// Tests the next triangle of a non-empty `leaf`; true when it was hit (and
+// is the closest hit so far, or for ANY_HIT ends the ray).
+template<bool ANY_HIT, bool EXACT_MT, int WT>
+DG_HD bool trav_tri(TravState& s, const TraceScene& sc, uint2& leaf) {
+  const uint32_t below = (leaf.y & (0u - leaf.y)) - 1u;
+  const uint32_t index = leaf.x + DG_POPC((leaf.y >> 16) & below);
+  leaf.y &= leaf.y - 1u;
+  const float4* tp = sc.tris + 3 * size_t(index);
+  float4 a = DG_LDG(tp), e1 = DG_LDG(tp + 1), e2 = DG_LDG(tp + 2);
+  float t, b1, b2;
+  bool h;
+  if(WT == kTriWatertight || (WT == kTriByScene && sc.watertight)) {
+    h = wt_hit(s.wt, a, e1, e2, s.ox, s.oy, s.oz, s.t_min, s.best.t, t, b1, b2);
+  } else {
+    h = EXACT_MT
+        ? mt_exact(a, e1, e2, s.ox, s.oy, s.oz, s.dx, s.dy, s.dz, s.t_min, s.best.t, t, b1, b2)
+        : mt_fast(a, e1, e2, s.ox, s.oy, s.oz, s.dx, s.dy, s.dz, s.t_min, s.best.t, t, b1, b2);
+  }
+  if(h) {
+    uint32_t id = DG_AS_UINT(a.w);
+    if(ANY_HIT || s.best.prim == kMiss || t < s.best.t || id > s.best.prim) {
+      s.best.t = t; s.best.b1 = b1; s.best.b2 = b2; s.best.prim = id;
+      return true;
     }
   }
-  return (s.group.y & 0xff000000u) == 0u && s.sp == 0;
+  return false;
+}
+
+// One traversal step; returns true when the ray is finished (s.best holds
+// the closest hit, or for ANY_HIT the first hit found, or prim = kMiss).
+template<bool ANY_HIT, bool EXACT_MT, class Stack, int WT = kTriMt>
+DG_HD bool trav_step(TravState& s, const TraceScene& sc, Stack& stack) {
+  if(!group_left(s)) { return true; }   // an empty tree
+  uint2 leaf = trav_node(s, sc, stack);
+  while(!leaf_empty(leaf)) {
+    if(trav_tri<ANY_HIT, EXACT_MT, WT>(s, sc, leaf) && ANY_HIT) { return true; }
+  }
+  return !group_left(s);
 }
 
 // Closest hit (ANY_HIT = false) or any hit (ANY_HIT = true) of one ray.

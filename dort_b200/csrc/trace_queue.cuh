@@ -1,0 +1,164 @@
+// Warp-cooperative traversal of a queue of rays (device only).
+//
+// One ray per thread inside a persistent warp, as in trace_ray, but the warp
+// decides together what its lanes do next, so that divergent rays keep the
+// lanes busy:
+//   - a lane whose ray is finished takes the queue's next ray as soon as
+//     kIdleLanes lanes are idle, instead of waiting for the warp's longest
+//     ray;
+//   - leaf triangles are not tested in the node step that finds them: a lane
+//     holds up to two nodes' worth of them and goes on with its nodes until
+//     kTriLanes lanes hold some (or fewer than kMinLanes can go on), and the
+//     warp then tests triangles together until fewer than kMinLanes hold any.
+// Neither changes a result: the closest hit is the minimum over the triangles
+// tested (ties go to the larger index), whatever their order; a later
+// triangle test only means that a few more boxes pass against the older t.
+//
+// Measured on the 1M-triangle soup: a warp's 32 diffuse bounce rays took 59
+// node steps with 16.5 lanes active and 115 triangle tests with 3.5 lanes
+// active one ray per lane to the end; 37.5 steps with 26 lanes and 34 tests
+// with 12 lanes this way (4M such rays: 3.61 ms against 2.47 ms; the camera
+// rays of the same scene 1.69 against 1.65 ms).
+#pragma once
+#include "trace.cuh"
+
+namespace dort_gpu {
+
+constexpr uint32_t kNoItem = 0xffffffffu;
+constexpr uint32_t kWarpAll = 0xffffffffu;
+
+constexpr int kTriLanes = 16;
+constexpr int kMinLanes = 8;
+constexpr int kIdleLanes = 4;
+
+// Entries of a queue that every warp starts with: an equal share of a short
+// queue, down to a single entry (a ray alone in its warp is finished
+// soonest), half of a longer one's, at most 64.
+__host__ __device__ __forceinline__ uint32_t queue_first(uint32_t count, uint32_t warps) {
+  const uint32_t share = count / warps + (count % warps ? 1u : 0u);
+  return share <= 16u ? (share ? share : 1u) : (share < 128u ? share / 2u : 64u);
+}
+
+// Entries a warp takes at a time after that when `left` are not yet taken:
+// fewer towards the queue's end, so that the warps finish together.
+__device__ __forceinline__ uint32_t queue_next(uint32_t left, uint32_t warps) {
+  return min(64u, max(8u, left / (4u * warps)));
+}
+
+// Entries of a queue's results that wait in shared memory until 32 of them
+// can be worked off by the whole warp (a finished ray's follow-up loads would
+// otherwise stall the warp for a few lanes).  kSlots words per warp.
+struct WarpBuffer {
+  static constexpr uint32_t kSlots = 64;
+  uint32_t* slots;     // this warp's words
+  uint32_t count;      // warp-uniform
+
+  // Adds `value` of every lane with `want`; true when 32 entries are there.
+  __device__ __forceinline__ bool push(bool want, uint32_t value) {
+    const uint32_t mask = __ballot_sync(kWarpAll, want);
+    const uint32_t lane = threadIdx.x & 31u;
+    if(want) { slots[count + __popc(mask & ((1u << lane) - 1u))] = value; }
+    count += __popc(mask);
+    return count >= 32u;
+  }
+  // This lane's entry of the 32 (or the last few) oldest, kNoItem if none.
+  __device__ __forceinline__ uint32_t take() {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    const uint32_t v = lane < count ? slots[lane] : kNoItem;
+    const uint32_t rest = lane + 32u < count ? slots[lane + 32u] : 0u;
+    __syncwarp();
+    if(lane + 32u < count) { slots[lane] = rest; }
+    count = count > 32u ? count - 32u : 0u;
+    return v;
+  }
+};
+
+// Traces the entries [0, count) of a queue.  Every warp starts with the chunk
+// of its own number; `cursor` (zero before) counts the entries taken after
+// those, and is left alone by queues that the first chunks cover.
+// Q:
+//   const TraceScene& scene()               the scene of this lane's ray
+//   void load(uint32_t i, TravState& s)     starts the ray of entry i
+//   void done(bool mine, uint32_t i, const TravState& s)
+//     called by the whole warp; lanes with `mine` have finished entry i (s.best)
+template<bool ANY_HIT, bool EXACT_MT, int WT, class Q>
+__device__ __forceinline__ void trace_queue(Q& q, uint32_t count, uint32_t* cursor) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t first = queue_first(count, warps);
+  // the warp's entries not yet started
+  uint32_t next = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * first;
+  uint32_t end = min(next + first, count);
+  bool more = warps * first < count;   // the cursor may have more
+  uint32_t item = kNoItem;        // this lane's entry
+  uint32_t idle = kWarpAll;       // lanes without one
+  TravState s;
+  s.group = make_uint2(0u, 0u);
+  s.sp = 0;
+  TraceStack stack;
+  stack.init();
+  uint2 leaf = make_uint2(0u, 0u), leaf2 = make_uint2(0u, 0u);   // triangles to test
+  for(;;) {
+    if(__popc(idle) >= kIdleLanes) {
+      if(next >= end && more) {
+        const uint32_t want = queue_next(count - end, warps);
+        uint32_t b = 0;
+        if(lane == 0) { b = atomicAdd(cursor, want); }
+        next = warps * first + __shfl_sync(kWarpAll, b, 0);
+        end = min(next + want, count);
+        more = next < count;
+      }
+      if(next < end) {
+        const uint32_t at = next + __popc(idle & lt);
+        if(item == kNoItem && at < end) {
+          item = at;
+          q.load(item, s);
+        }
+        next += __popc(idle);
+      } else if(idle == kWarpAll) {
+        break;
+      }
+    }
+    // node steps; a lane with two nodes' triangles waits
+    for(;;) {
+      if(group_left(s) && leaf_empty(leaf2)) {
+        const uint2 l = trav_node(s, q.scene(), stack);
+        if(!leaf_empty(l)) {
+          leaf2 = leaf;
+          leaf = l;
+        }
+      }
+      const uint32_t tri = __ballot_sync(kWarpAll, !leaf_empty(leaf));
+      if(__popc(tri) >= kTriLanes) { break; }
+      const uint32_t node = __ballot_sync(kWarpAll, group_left(s) && leaf_empty(leaf2));
+      if(__popc(node) < kMinLanes) { break; }
+      if(more && __popc(node | tri) <= 32 - kIdleLanes) { break; }
+    }
+    // triangle tests, one per lane and round
+    uint32_t tri;
+    do {
+      if(!leaf_empty(leaf)) {
+        if(trav_tri<ANY_HIT, EXACT_MT, WT>(s, q.scene(), leaf) && ANY_HIT) {
+          leaf.y = 0u;
+          leaf2.y = 0u;
+          s.group.y = 0u;
+          s.sp = 0;
+        }
+        if(leaf_empty(leaf)) {
+          leaf = leaf2;
+          leaf2.y = 0u;
+        }
+      }
+      tri = __ballot_sync(kWarpAll, !leaf_empty(leaf));
+    } while(__popc(tri) >= kMinLanes);
+    const bool mine = item != kNoItem && !group_left(s) && leaf_empty(leaf);
+    if(__any_sync(kWarpAll, mine)) {
+      q.done(mine, item, s);
+      if(mine) { item = kNoItem; }
+    }
+    idle = __ballot_sync(kWarpAll, item == kNoItem);
+  }
+}
+
+}  // namespace dort_gpu

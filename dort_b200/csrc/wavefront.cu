@@ -33,6 +33,7 @@
 #include "common.h"
 #include "pt.cuh"
 #include "scene_build.h"
+#include "trace_queue.cuh"
 #include "wavefront.h"
 
 namespace dort_gpu {
@@ -558,52 +559,118 @@ __global__ void wf_classify(WfDev w) {
   }
 }
 
-// Register cap of the trace stages (extend, shadow): 56 instead of the 64
-// the compiler picks (a few bytes of spill) lets 9 instead of 8 blocks of 128
-// threads share an SM; the 1080p frame measured 659.7 against 652.2 M
-// samples/s (extend 338.9 against 345.4 ms).
+// Register cap of the trace stages (extend, shadow, neeb): 8 blocks of 128
+// threads per SM.
 #ifndef DORT_TRACE_MAXNREG
-#define DORT_TRACE_MAXNREG 56
+#define DORT_TRACE_MAXNREG 64
 #endif
 #define DORT_TRACE_REGS __maxnreg__(DORT_TRACE_MAXNREG)
 
+// The scene of the ray a lane traces: the frame's, or in a batch the job's
+// (kept per lane, since a warp's rays may belong to several jobs).
+template<class J, bool kBatched = J::kBatched>
+struct LaneScene {
+  const PtScene* sc;
+  __device__ __forceinline__ explicit LaneScene(const J& jobs) : sc(&jobs.scene(0)) {}
+  __device__ __forceinline__ void select(const J&, const WfDev&, uint32_t) {}
+  __device__ __forceinline__ const PtScene& pt() const { return *sc; }
+  __device__ __forceinline__ const TraceScene& trace() const { return sc->trace; }
+};
 template<class J>
-__global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
-  const uint32_t cur = wave_of(w) & 1u;
-  const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_ACT0 + cur);
-  const uint32_t* act = w.sorted ? w.sort_val[1] : w.active[cur];
-  for(;;) {
-    uint32_t base = warp_fetch(ctr_at(w.ctr, C_F_EXT));
-    if(base >= n) { break; }
-    uint32_t i = base + (threadIdx.x & 31u);
-    uint32_t slot = 0, kind = kShadeQueues;
-    if(i < n) {
-      slot = act[i];
-      uint32_t job = J::kBatched ? (w.meta[slot].w >> 8) : 0u;
-      const PtScene& sc = jobs.scene(job);
-      float4 o = w.ray_o[slot], d = w.ray_d[slot];
-      Hit h = scene_trace<false, J::kGeneral>(sc, v3(o.x, o.y, o.z), o.w, v3(d.x, d.y, d.z),
-                                              INFINITY);
+struct LaneScene<J, true> {
+  const PtScene* sc;
+  TraceScene tr;
+  __device__ __forceinline__ explicit LaneScene(const J& jobs)
+      : sc(&jobs.scene(0)), tr(sc->trace) {}
+  __device__ __forceinline__ void select(const J& jobs, const WfDev& w, uint32_t slot) {
+    sc = &jobs.scene(w.meta[slot].w >> 8);
+    tr = sc->trace;
+  }
+  __device__ __forceinline__ const PtScene& pt() const { return *sc; }
+  __device__ __forceinline__ const TraceScene& trace() const { return tr; }
+};
+
+// A finished triangle traversal with the scene's analytic shapes tested too.
+template<bool ANY_HIT, bool G>
+__device__ __forceinline__ Hit with_shapes(const PtScene& sc, const TravState& s, float t_max) {
+  if(!G || sc.shape_count == 0 || (ANY_HIT && s.best.prim != kMiss)) { return s.best; }
+  return trace_shapes<ANY_HIT>(sc, v3(s.ox, s.oy, s.oz), s.t_min, v3(s.dx, s.dy, s.dz), t_max,
+                               s.best);
+}
+
+template<bool G>
+constexpr int kTraceTest = G ? kTriByScene : kTriMt;
+
+// The extension queue: closest hit of each active path; the finished paths
+// wait in shared memory until 32 of them can be sorted into the shade queues
+// together (one atomic per warp and kind, and one wait for their materials).
+template<class J>
+struct ExtendQueue {
+  const J& jobs;
+  WfDev& w;
+  const uint32_t* act;
+  LaneScene<J> scene_of;
+  uint32_t slot = 0;
+  WarpBuffer buf;
+  __device__ __forceinline__ const TraceScene& scene() const { return scene_of.trace(); }
+  __device__ __forceinline__ void load(uint32_t i, TravState& s) {
+    slot = act[i];
+    scene_of.select(jobs, w, slot);
+    const float4 o = w.ray_o[slot], d = w.ray_d[slot];
+    trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, INFINITY);
+  }
+  __device__ __forceinline__ void done(bool mine, uint32_t, const TravState& s) {
+    if(mine) {
+      const Hit h = with_shapes<false, J::kGeneral>(scene_of.pt(), s, INFINITY);
       w.hit[slot] = make_float4(h.t, h.b1, h.b2, u2f(h.prim));
+    }
+    if(buf.push(mine, slot)) { classify(); }
+  }
+  __device__ __forceinline__ void classify() {
+    const uint32_t sl = buf.take();
+    uint32_t kind = kShadeQueues;
+    if(sl != kNoItem) {
       kind = kMissQueue;
-      if(h.prim != kMiss) {
-        uint32_t mat = prim_material<J::kGeneral>(sc, h.prim);
+      const uint32_t prim = f2u(__ldcg(&w.hit[sl].w));
+      if(prim != kMiss) {
+        const PtScene& sc = jobs.scene(J::kBatched ? (w.meta[sl].w >> 8) : 0u);
+        uint32_t mat = prim_material<J::kGeneral>(sc, prim);
         kind = __ldg(&sc.mats[mat].kind);
         // Oren-Nayar shares the Lambert queue (the queues only group work)
         if(kind >= kMissQueue) { kind = DORT_MAT_LAMBERT; }
       }
     }
     if(w.sorted) {
-      if(i < n) { w.hit_kind[slot] = kind; }
-      continue;
+      if(sl != kNoItem) { w.hit_kind[sl] = kind; }
+      return;
     }
 #pragma unroll
     for(uint32_t k = 0; k < kShadeQueues; ++k) {
       bool mine = kind == k;
       uint32_t at = warp_append(ctr_at(w.ctr, C_KQ0 + k), mine);
-      if(mine) { w.kq[k][at] = slot; }
+      if(mine) { w.kq[k][at] = sl; }
     }
   }
+};
+
+// Shared memory of a trace stage: every warp's WarpBuffer.
+static size_t trace_shared_bytes(int block) {
+  return size_t(block / 32) * WarpBuffer::kSlots * sizeof(uint32_t);
+}
+
+__device__ __forceinline__ WarpBuffer warp_buffer() {
+  extern __shared__ uint32_t trace_slots[];
+  return WarpBuffer{trace_slots + (threadIdx.x >> 5) * WarpBuffer::kSlots, 0u};
+}
+
+template<class J>
+__global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
+  const uint32_t cur = wave_of(w) & 1u;
+  const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_ACT0 + cur);
+  ExtendQueue<J> q{jobs, w, w.sorted ? w.sort_val[1] : w.active[cur], LaneScene<J>(jobs), 0u,
+                   warp_buffer()};
+  trace_queue<false, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_EXT));
+  if(q.buf.count) { q.classify(); }
 }
 
 // The direct lighting of one light at a path vertex (estimate_direct,
@@ -870,30 +937,52 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w) {
   }
 }
 
-// One shadow-queue entry: any hit of its segment; if nothing blocks it, its
-// contribution joins its path's sum.
+// A shadow-queue entry that nothing blocks: its contribution joins its path's
+// sum.
 template<class J>
-__device__ __forceinline__ void shadow_entry(J& jobs, WfDev& w, uint32_t i, float4 o, float4 d) {
-  uint32_t slot = w.sh_slot[i];
-  uint32_t job = J::kBatched ? (w.meta[slot].w >> 8) : 0u;
-  const PtScene& sc = jobs.scene(job);
-  Hit h = scene_trace<true, J::kGeneral>(sc, v3(o.x, o.y, o.z), o.w, v3(d.x, d.y, d.z), d.w);
-  if(h.prim == kMiss) {
-    // a path can own two entries (light and BSDF strategy for a background
-    // light), so the additions are atomic
-    float4 c = w.sh_c[i];
-    float* sp = &w.sum[slot].x;
-    atomicAdd(sp, c.x);
-    atomicAdd(sp + 1, c.y);
-    atomicAdd(sp + 2, c.z);
-    if constexpr(J::kAdjoint) {
-      const uint32_t light_tri = f2u(c.w);
-      if(jobs.d_emission && light_tri != kMiss) {
-        adj_record<true>(w, slot, kEvDirect, light_tri, v3(c.x, c.y, c.z));
-      }
+__device__ __forceinline__ void shadow_add(const J& jobs, WfDev& w, uint32_t i) {
+  // a path can own two entries (light and BSDF strategy for a background
+  // light), so the additions are atomic
+  const uint32_t slot = w.sh_slot[i];
+  float4 c = w.sh_c[i];
+  float* sp = &w.sum[slot].x;
+  atomicAdd(sp, c.x);
+  atomicAdd(sp + 1, c.y);
+  atomicAdd(sp + 2, c.z);
+  if constexpr(J::kAdjoint) {
+    const uint32_t light_tri = f2u(c.w);
+    if(jobs.d_emission && light_tri != kMiss) {
+      adj_record<true>(w, slot, kEvDirect, light_tri, v3(c.x, c.y, c.z));
     }
   }
 }
+
+// The shadow queue: any hit of each entry's segment; the entries that nothing
+// blocks wait in shared memory until 32 of them are added together.
+template<class J>
+struct ShadowQueue {
+  const J& jobs;
+  WfDev& w;
+  LaneScene<J> scene_of;
+  float t_max = 0.f;
+  WarpBuffer buf;
+  __device__ __forceinline__ const TraceScene& scene() const { return scene_of.trace(); }
+  __device__ __forceinline__ void load(uint32_t i, TravState& s) {
+    if(J::kBatched) { scene_of.select(jobs, w, w.sh_slot[i]); }
+    const float4 o = w.sh_o[i], d = w.sh_d[i];
+    t_max = d.w;
+    trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, d.w);
+  }
+  __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) {
+    const bool open = mine &&
+                      with_shapes<true, J::kGeneral>(scene_of.pt(), s, t_max).prim == kMiss;
+    if(buf.push(open, i)) { add(); }
+  }
+  __device__ __forceinline__ void add() {
+    const uint32_t i = buf.take();
+    if(i != kNoItem) { shadow_add(jobs, w, i); }
+  }
+};
 
 // Staging of the shadow queue through the bulk-copy (TMA) engine.  The queue
 // is contiguous in entry order, so a warp's next 32 entries (origins and
@@ -983,74 +1072,84 @@ __global__ void DORT_TRACE_REGS wf_shadow(J jobs, WfDev w) {
       if(next < n && lane == 0) {
         stage_batch(st, &bar[warp], w.sh_o + next, w.sh_d + next, min(32u, n - next));
       }
-      if(i < n) { shadow_entry(jobs, w, i, o, d); }
+      if(i < n) {
+        const PtScene& sc = jobs.scene(J::kBatched ? (w.meta[w.sh_slot[i]].w >> 8) : 0u);
+        Hit h = scene_trace<true, J::kGeneral>(sc, v3(o.x, o.y, o.z), o.w, v3(d.x, d.y, d.z),
+                                               d.w);
+        if(h.prim == kMiss) { shadow_add(jobs, w, i); }
+      }
       base = next;
     }
     return;
   }
-  for(;;) {
-    uint32_t base = warp_fetch(ctr_at(w.ctr, C_F_SH));
-    if(base >= n) { break; }
-    uint32_t i = base + lane;
-    if(i < n) { shadow_entry(jobs, w, i, w.sh_o[i], w.sh_d[i]); }
-  }
+  ShadowQueue<J> q{jobs, w, LaneScene<J>(jobs), 0.f, warp_buffer()};
+  trace_queue<true, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_SH));
+  if(q.buf.count) { q.add(); }
 }
 
-template<bool G, bool ADJ>
-__device__ __forceinline__ void neeb_one_impl(const PtScene& sc, WfDev& w, uint32_t i,
-                                              bool want_emission);
+// Light of a hit primitive (index + 1, 0: none).
+template<bool G>
+__device__ __forceinline__ uint32_t prim_light(const PtScene& sc, uint32_t prim) {
+  if(G && prim >= sc.shape_base) { return sc.shapes[prim - sc.shape_base].light; }
+  return DG_AS_UINT(DG_LDG(&sc.shade[3 * size_t(prim) + 1].w));
+}
+
+// The BSDF-strategy queue: rays towards area lights, which count when their
+// closest hit is the light's own primitive.
+template<class J>
+struct NeebQueue {
+  const J& jobs;
+  WfDev& w;
+  LaneScene<J> scene_of;
+  __device__ __forceinline__ const TraceScene& scene() const { return scene_of.trace(); }
+  __device__ __forceinline__ void load(uint32_t i, TravState& s) {
+    if(J::kBatched) { scene_of.select(jobs, w, w.nb_slot[i]); }
+    const float4 o = w.nb_o[i], d = w.nb_d[i];
+    trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, INFINITY);
+  }
+  __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) {
+    if(!mine) { return; }
+    const PtScene& sc = scene_of.pt();
+    const Hit h = with_shapes<false, J::kGeneral>(sc, s, INFINITY);
+    if(h.prim == kMiss) { return; }
+    const uint32_t lw = f2u(w.nb_f[i].w);
+    if(prim_light<J::kGeneral>(sc, h.prim) == (lw & 0x7fffffffu) + 1u) { add(sc, i, h); }
+  }
+  __device__ __forceinline__ void add(const PtScene& sc, uint32_t i, const Hit& h) {
+    constexpr bool G = J::kGeneral;
+    const float4 o = w.nb_o[i], d = w.nb_d[i], f = w.nb_f[i];
+    const uint32_t lw = f2u(f.w), li = lw & 0x7fffffffu;
+    const bool use_mis = (lw >> 31) != 0;
+    const DevLight& l = sc.lights[li];
+    const V3 p = v3(o.x, o.y, o.z), wi = v3(d.x, d.y, d.z);
+    const V3 L = area_light_hit_radiance<G>(sc, li, h, p, wi);
+    if(is_black(L)) { return; }
+    float wgt = 1.f;
+    if(use_mis) {
+      float lp = light_pivot_pdf<G>(sc, l, wi, p);
+      wgt = d.w / (d.w + lp);
+    }
+    V3 c = v3(f.x, f.y, f.z) * L * wgt;
+    // with sample_all_lights a path owns one entry per area light, which
+    // may run in the same wave of this kernel: the additions are atomic
+    const uint32_t slot = w.nb_slot[i];
+    float* sp = &w.sum[slot].x;
+    atomicAdd(sp, c.x);
+    atomicAdd(sp + 1, c.y);
+    atomicAdd(sp + 2, c.z);
+    if constexpr(J::kAdjoint) {
+      if(jobs.d_emission && l.kind == LIGHT_TRI) {
+        adj_record<true>(w, slot, kEvDirect, l.tri, c);
+      }
+    }
+  }
+};
 
 template<class J>
-__global__ void wf_neeb(J jobs, WfDev w) {
+__global__ void DORT_TRACE_REGS wf_neeb(J jobs, WfDev w) {
   const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_NEEB);
-  for(;;) {
-    uint32_t base = warp_fetch(ctr_at(w.ctr, C_F_NB));
-    if(base >= n) { break; }
-    uint32_t i = base + (threadIdx.x & 31u);
-    if(i < n) {
-      uint32_t job = J::kBatched ? (w.meta[w.nb_slot[i]].w >> 8) : 0u;
-      bool want_emission = false;
-      if constexpr(J::kAdjoint) { want_emission = jobs.d_emission != nullptr; }
-      neeb_one_impl<J::kGeneral, J::kAdjoint>(jobs.scene(job), w, i, want_emission);
-    }
-  }
-}
-
-template<bool G, bool ADJ>
-__device__ __forceinline__ void neeb_one_impl(const PtScene& sc, WfDev& w, uint32_t i,
-                                              bool want_emission) {
-    float4 o = w.nb_o[i], d = w.nb_d[i], f = w.nb_f[i];
-    uint32_t lw = f2u(f.w);
-    const uint32_t li = lw & 0x7fffffffu;
-    const DevLight& l = sc.lights[li];
-    bool use_mis = (lw >> 31) != 0;
-    V3 L = v3(0.f, 0.f, 0.f);
-    V3 p = v3(o.x, o.y, o.z), wi = v3(d.x, d.y, d.z);
-    if(light_is_area(l)) {
-      Hit h = scene_trace<false, G>(sc, p, o.w, wi, INFINITY);
-      L = area_light_hit_radiance<G>(sc, li, h, p, wi);
-    } else {
-      // background light: only escaping rays count, an any-hit query decides
-      Hit h = scene_trace<true, G>(sc, p, o.w, wi, INFINITY);
-      if(h.prim == kMiss) { L = background_radiance(sc, l, wi); }
-    }
-    if(!is_black(L)) {
-      float wgt = 1.f;
-      if(use_mis) {
-        float lp = light_pivot_pdf<G>(sc, l, wi, p);
-        wgt = d.w / (d.w + lp);
-      }
-      V3 c = v3(f.x, f.y, f.z) * L * wgt;
-      // with sample_all_lights a path owns one entry per area light, which
-      // may run in the same wave of this kernel: the additions are atomic
-      float* sp = &w.sum[w.nb_slot[i]].x;
-      atomicAdd(sp, c.x);
-      atomicAdd(sp + 1, c.y);
-      atomicAdd(sp + 2, c.z);
-      if(ADJ && want_emission && l.kind == LIGHT_TRI) {
-        adj_record<true>(w, w.nb_slot[i], kEvDirect, l.tri, c);
-      }
-    }
+  NeebQueue<J> q{jobs, w, LaneScene<J>(jobs)};
+  trace_queue<false, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_NB));
 }
 
 // Single thread: account the wave, retire its queues, decide whether to loop.
@@ -1241,11 +1340,11 @@ static int wf_alloc(Wavefront* wf, uint32_t capacity, uint32_t npix, uint32_t ne
   return DORT_OK;
 }
 
-static int grid_for(const void* kernel, int block) {
+static int grid_for(const void* kernel, int block, size_t shared = 0) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, shared);
   return sms * std::max(per_sm, 1);
 }
 
@@ -1279,9 +1378,9 @@ static WfGrids wf_grids(const WfTuning& tn) {
   g.b_shw = fit_block(shw, int(tn.trace_block));
   g.b_nb = fit_block(nb, int(tn.trace_block));
   g.regen = grid_for(reinterpret_cast<const void*>(&wf_regen<J>), int(kRegenBlock));
-  g.ext = grid_for(ext, g.b_ext);
+  g.ext = grid_for(ext, g.b_ext, trace_shared_bytes(g.b_ext));
   g.sha = grid_for(sha, g.b_sha);
-  g.shw = grid_for(shw, g.b_shw);
+  g.shw = grid_for(shw, g.b_shw, trace_shared_bytes(g.b_shw));
   g.nb = grid_for(nb, g.b_nb);
   return g;
 }
@@ -1302,7 +1401,7 @@ template<class J>
 static void wf_launch_extend(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
                              cudaStream_t st) {
   if(tn.sort) { wf_sort<J>(jobs, dev, g, st); }
-  wf_extend<J><<<g.ext, g.b_ext, 0, st>>>(jobs, dev);
+  wf_extend<J><<<g.ext, g.b_ext, trace_shared_bytes(g.b_ext), st>>>(jobs, dev);
   if(tn.sort) { wf_classify<<<g.regen, 256, 0, st>>>(dev); }
 }
 
@@ -1310,9 +1409,9 @@ template<class J>
 static void wf_launch_shadow(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
                              cudaStream_t st) {
   if(tn.stage_queues) {
-    wf_shadow<J, true><<<g.shw, g.b_shw, 0, st>>>(jobs, dev);
+    wf_shadow<J, true><<<g.shw, g.b_shw, trace_shared_bytes(g.b_shw), st>>>(jobs, dev);
   } else {
-    wf_shadow<J, false><<<g.shw, g.b_shw, 0, st>>>(jobs, dev);
+    wf_shadow<J, false><<<g.shw, g.b_shw, trace_shared_bytes(g.b_shw), st>>>(jobs, dev);
   }
 }
 
