@@ -33,44 +33,65 @@ constexpr int kIdleLanes = 4;
 
 // Entries of a queue that every warp starts with: an equal share of a short
 // queue, down to a single entry (a ray alone in its warp is finished
-// soonest), half of a longer one's, at most 64.
+// soonest), 64 of a long one.
 __host__ __device__ __forceinline__ uint32_t queue_first(uint32_t count, uint32_t warps) {
   const uint32_t share = count / warps + (count % warps ? 1u : 0u);
-  return share <= 16u ? (share ? share : 1u) : (share < 128u ? share / 2u : 64u);
+  return share < 1u ? 1u : (share > 64u ? 64u : share);
 }
 
 // Entries a warp takes at a time after that when `left` are not yet taken:
-// fewer towards the queue's end, so that the warps finish together.
+// half a share towards the queue's end, so that the warps finish together,
+// but not so few that the cursor's atomics (about 1 ns each, one address) add
+// up: with eighths down to 8 entries the Cornell frame took 3.92 ms instead
+// of 3.65.
 __device__ __forceinline__ uint32_t queue_next(uint32_t left, uint32_t warps) {
-  return min(64u, max(8u, left / (4u * warps)));
+  return min(64u, max(16u, left / (2u * warps)));
 }
 
-// Entries of a queue's results that wait in shared memory until 32 of them
-// can be worked off by the whole warp (a finished ray's follow-up loads would
-// otherwise stall the warp for a few lanes).  kSlots words per warp.
+// Results that wait in shared memory until 32 of them can be worked off by
+// the whole warp (a finished ray's follow-up loads would otherwise stall the
+// warp for a few lanes).  kSlots entries of kWords words per warp.
+template<uint32_t kWords>
 struct WarpBuffer {
   static constexpr uint32_t kSlots = 64;
   uint32_t* slots;     // this warp's words
   uint32_t count;      // warp-uniform
 
-  // Adds `value` of every lane with `want`; true when 32 entries are there.
-  __device__ __forceinline__ bool push(bool want, uint32_t value) {
+  static constexpr size_t bytes(int block) {
+    return size_t(block / 32) * kSlots * kWords * sizeof(uint32_t);
+  }
+  __device__ __forceinline__ static WarpBuffer of_warp(uint32_t* shared) {
+    return WarpBuffer{shared + (threadIdx.x >> 5) * kSlots * kWords, 0u};
+  }
+  // Adds the entry (a, b) of every lane with `want` (b with two words); true
+  // when 32 entries are there.
+  __device__ __forceinline__ bool push(bool want, uint32_t a, uint32_t b = 0u) {
     const uint32_t mask = __ballot_sync(kWarpAll, want);
     const uint32_t lane = threadIdx.x & 31u;
-    if(want) { slots[count + __popc(mask & ((1u << lane) - 1u))] = value; }
+    if(want) {
+      const uint32_t at = count + __popc(mask & ((1u << lane) - 1u));
+      slots[at] = a;
+      if(kWords > 1) { slots[at + kSlots] = b; }
+    }
     count += __popc(mask);
     return count >= 32u;
   }
-  // This lane's entry of the 32 (or the last few) oldest, kNoItem if none.
-  __device__ __forceinline__ uint32_t take() {
+  // This lane's entry of the 32 (or the last few) oldest; false if none.
+  __device__ __forceinline__ bool take(uint32_t& a, uint32_t& b) {
     const uint32_t lane = threadIdx.x & 31u;
+    const bool have = lane < count, rest = lane + 32u < count;
     __syncwarp();
-    const uint32_t v = lane < count ? slots[lane] : kNoItem;
-    const uint32_t rest = lane + 32u < count ? slots[lane + 32u] : 0u;
+    a = slots[lane];
+    b = kWords > 1 ? slots[lane + kSlots] : 0u;
+    const uint32_t ra = slots[lane + 32u];
+    const uint32_t rb = kWords > 1 ? slots[lane + 32u + kSlots] : 0u;
     __syncwarp();
-    if(lane + 32u < count) { slots[lane] = rest; }
+    if(rest) {
+      slots[lane] = ra;
+      if(kWords > 1) { slots[lane + kSlots] = rb; }
+    }
     count = count > 32u ? count - 32u : 0u;
-    return v;
+    return have;
   }
 };
 

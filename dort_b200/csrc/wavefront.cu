@@ -611,7 +611,7 @@ struct ExtendQueue {
   const uint32_t* act;
   LaneScene<J> scene_of;
   uint32_t slot = 0;
-  WarpBuffer buf;
+  WarpBuffer<2> buf;   // slot, hit primitive
   __device__ __forceinline__ const TraceScene& scene() const { return scene_of.trace(); }
   __device__ __forceinline__ void load(uint32_t i, TravState& s) {
     slot = act[i];
@@ -620,18 +620,19 @@ struct ExtendQueue {
     trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, INFINITY);
   }
   __device__ __forceinline__ void done(bool mine, uint32_t, const TravState& s) {
+    uint32_t prim = kMiss;
     if(mine) {
       const Hit h = with_shapes<false, J::kGeneral>(scene_of.pt(), s, INFINITY);
       w.hit[slot] = make_float4(h.t, h.b1, h.b2, u2f(h.prim));
+      prim = h.prim;
     }
-    if(buf.push(mine, slot)) { classify(); }
+    if(buf.push(mine, slot, prim)) { classify(); }
   }
   __device__ __forceinline__ void classify() {
-    const uint32_t sl = buf.take();
-    uint32_t kind = kShadeQueues;
-    if(sl != kNoItem) {
+    uint32_t sl, prim, kind = kShadeQueues;
+    const bool have = buf.take(sl, prim);
+    if(have) {
       kind = kMissQueue;
-      const uint32_t prim = f2u(__ldcg(&w.hit[sl].w));
       if(prim != kMiss) {
         const PtScene& sc = jobs.scene(J::kBatched ? (w.meta[sl].w >> 8) : 0u);
         uint32_t mat = prim_material<J::kGeneral>(sc, prim);
@@ -641,7 +642,7 @@ struct ExtendQueue {
       }
     }
     if(w.sorted) {
-      if(sl != kNoItem) { w.hit_kind[sl] = kind; }
+      if(have) { w.hit_kind[sl] = kind; }
       return;
     }
 #pragma unroll
@@ -653,22 +654,14 @@ struct ExtendQueue {
   }
 };
 
-// Shared memory of a trace stage: every warp's WarpBuffer.
-static size_t trace_shared_bytes(int block) {
-  return size_t(block / 32) * WarpBuffer::kSlots * sizeof(uint32_t);
-}
-
-__device__ __forceinline__ WarpBuffer warp_buffer() {
-  extern __shared__ uint32_t trace_slots[];
-  return WarpBuffer{trace_slots + (threadIdx.x >> 5) * WarpBuffer::kSlots, 0u};
-}
+extern __shared__ uint32_t trace_shared[];   // the trace stages' WarpBuffers
 
 template<class J>
 __global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
   const uint32_t cur = wave_of(w) & 1u;
   const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_ACT0 + cur);
   ExtendQueue<J> q{jobs, w, w.sorted ? w.sort_val[1] : w.active[cur], LaneScene<J>(jobs), 0u,
-                   warp_buffer()};
+                   WarpBuffer<2>::of_warp(trace_shared)};
   trace_queue<false, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_EXT));
   if(q.buf.count) { q.classify(); }
 }
@@ -965,7 +958,7 @@ struct ShadowQueue {
   WfDev& w;
   LaneScene<J> scene_of;
   float t_max = 0.f;
-  WarpBuffer buf;
+  WarpBuffer<1> buf;   // entry
   __device__ __forceinline__ const TraceScene& scene() const { return scene_of.trace(); }
   __device__ __forceinline__ void load(uint32_t i, TravState& s) {
     if(J::kBatched) { scene_of.select(jobs, w, w.sh_slot[i]); }
@@ -979,8 +972,8 @@ struct ShadowQueue {
     if(buf.push(open, i)) { add(); }
   }
   __device__ __forceinline__ void add() {
-    const uint32_t i = buf.take();
-    if(i != kNoItem) { shadow_add(jobs, w, i); }
+    uint32_t i, unused;
+    if(buf.take(i, unused)) { shadow_add(jobs, w, i); }
   }
 };
 
@@ -1082,7 +1075,7 @@ __global__ void DORT_TRACE_REGS wf_shadow(J jobs, WfDev w) {
     }
     return;
   }
-  ShadowQueue<J> q{jobs, w, LaneScene<J>(jobs), 0.f, warp_buffer()};
+  ShadowQueue<J> q{jobs, w, LaneScene<J>(jobs), 0.f, WarpBuffer<1>::of_warp(trace_shared)};
   trace_queue<true, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_SH));
   if(q.buf.count) { q.add(); }
 }
@@ -1378,9 +1371,9 @@ static WfGrids wf_grids(const WfTuning& tn) {
   g.b_shw = fit_block(shw, int(tn.trace_block));
   g.b_nb = fit_block(nb, int(tn.trace_block));
   g.regen = grid_for(reinterpret_cast<const void*>(&wf_regen<J>), int(kRegenBlock));
-  g.ext = grid_for(ext, g.b_ext, trace_shared_bytes(g.b_ext));
+  g.ext = grid_for(ext, g.b_ext, WarpBuffer<2>::bytes(g.b_ext));
   g.sha = grid_for(sha, g.b_sha);
-  g.shw = grid_for(shw, g.b_shw, trace_shared_bytes(g.b_shw));
+  g.shw = grid_for(shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw));
   g.nb = grid_for(nb, g.b_nb);
   return g;
 }
@@ -1401,7 +1394,7 @@ template<class J>
 static void wf_launch_extend(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
                              cudaStream_t st) {
   if(tn.sort) { wf_sort<J>(jobs, dev, g, st); }
-  wf_extend<J><<<g.ext, g.b_ext, trace_shared_bytes(g.b_ext), st>>>(jobs, dev);
+  wf_extend<J><<<g.ext, g.b_ext, WarpBuffer<2>::bytes(g.b_ext), st>>>(jobs, dev);
   if(tn.sort) { wf_classify<<<g.regen, 256, 0, st>>>(dev); }
 }
 
@@ -1409,9 +1402,9 @@ template<class J>
 static void wf_launch_shadow(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
                              cudaStream_t st) {
   if(tn.stage_queues) {
-    wf_shadow<J, true><<<g.shw, g.b_shw, trace_shared_bytes(g.b_shw), st>>>(jobs, dev);
+    wf_shadow<J, true><<<g.shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw), st>>>(jobs, dev);
   } else {
-    wf_shadow<J, false><<<g.shw, g.b_shw, trace_shared_bytes(g.b_shw), st>>>(jobs, dev);
+    wf_shadow<J, false><<<g.shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw), st>>>(jobs, dev);
   }
 }
 

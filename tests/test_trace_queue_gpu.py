@@ -55,7 +55,7 @@ def test_queue_sizes_against_host(watertight):
     w = warps_of()
     # a lone ray, part of a warp, one ray per warp, the shares where the first
     # chunk changes, the first sizes that use the cursor, several chunks
-    sizes = sorted({1, 3, 31, 32, 33, w - 1, w, w + 1, 16 * w, 16 * w + 1, 24 * w + 5, 40 * w + 31})
+    sizes = sorted({1, 3, 31, 32, 33, w - 1, w, w + 1, 16 * w + 1, 64 * w, 64 * w + 1, 80 * w + 31})
     rays = random_rays(sizes[-1], 11)
     sc = db.Scene(verts, tris, watertight=watertight)
     ref, ref_tb, _ = db.host_check_raycast(verts, tris, rays, watertight=watertight)
