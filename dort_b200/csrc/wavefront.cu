@@ -8,13 +8,15 @@
 //   shade   emission, direct-lighting setup (one shadow ray and one
 //           BSDF-strategy ray per path into two queues), continuation
 //           sample, Russian roulette
-//   shadow  any hit of the shadow queue; unoccluded contributions added
-//   neeb    closest hit of the BSDF-strategy queue; light hits added with
+//   light   any hit of the shadow queue, unoccluded contributions added; then
+//           the closest hit of the BSDF-strategy queue, light hits added with
 //           their MIS weight
-//   control resets the queue counters and sets the loop condition
 //
 // The waves run inside one CUDA graph per frame: a conditional while node
-// whose body holds the six kernels, so the host launches a frame once.
+// whose body holds the four kernels, so the host launches a frame once.  The
+// loop condition is known after regen (extend notes it, shade sets it); the queue
+// counters are reset by the next kernel that does not use them (wave_begin,
+// wave_end).
 // Queues are compacted with warp ballots (one atomic per warp).  Every kernel
 // is a grid-stride loop over a count it reads from device memory, so the
 // graph's launch shapes are fixed.
@@ -48,6 +50,7 @@ enum : uint32_t {
   C_SHADOW = 4, C_NEEB = 5,    // this wave's shadow / BSDF-strategy queues
   C_LIVE = 6, C_WAVES = 7, C_ERROR = 8,
   C_F_EXT = 9, C_F_SHADE = 10, C_F_SH = 11, C_F_NB = 12,   // work-fetch cursors
+  C_MORE = 13,      // whether another wave follows
   C_KQ0 = 20,       // [20..25]: lengths of the shade queues by material kind
   C_NEXT_LO = 16,   // 64-bit next-sample counter at [16..17]
   C_RAYS_LO = 18,   // 64-bit ray counter at [18..19]
@@ -656,8 +659,43 @@ struct ExtendQueue {
 
 extern __shared__ uint32_t trace_shared[];   // the trace stages' WarpBuffers
 
+// One thread of extend: the lists that this wave's regen read are consumed,
+// the direct-lighting queues of the previous wave too; C_MORE says whether
+// another wave follows this one.
+__device__ __forceinline__ void wave_begin(WfDev& w) {
+  const uint32_t wave = wave_of(w), cur = wave & 1u;
+  *ctr_at(w.ctr, C_ACT0 + (cur ^ 1u)) = 0u;
+  *ctr_at(w.ctr, C_FIN0 + cur) = 0u;
+  *ctr_at(w.ctr, C_SHADOW) = 0u;
+  *ctr_at(w.ctr, C_NEEB) = 0u;
+  *ctr_at(w.ctr, C_F_SH) = 0u;
+  *ctr_at(w.ctr, C_F_NB) = 0u;
+  const uint64_t next = *reinterpret_cast<uint64_t*>(ctr_at(w.ctr, C_NEXT_LO));
+  bool more = *ctr_at(w.ctr, C_LIVE) > 0u || next < w.total_samples;
+  if(more && wave + 1u >= w.max_waves) {
+    // bounded: a frame never loops forever; the host reports the error
+    atomicOr(ctr_at(w.ctr, C_ERROR), 1u);
+    more = false;
+  }
+  *ctr_at(w.ctr, C_MORE) = more ? 1u : 0u;
+}
+
+// One thread of the wave's last kernel: the wave's rays are counted, the shade
+// queues consumed.  (Its own queues stay until the next wave_begin.)
+__device__ __forceinline__ void wave_end(WfDev& w) {
+  const uint32_t wave = wave_of(w);
+  unsigned long long* rays = reinterpret_cast<unsigned long long*>(ctr_at(w.ctr, C_RAYS_LO));
+  *rays += (unsigned long long)*ctr_at(w.ctr, C_ACT0 + (wave & 1u)) +
+           *ctr_at(w.ctr, C_SHADOW) + *ctr_at(w.ctr, C_NEEB);
+  *ctr_at(w.ctr, C_F_EXT) = 0u;
+  *ctr_at(w.ctr, C_F_SHADE) = 0u;
+  for(uint32_t k = 0; k < kShadeQueues; ++k) { *ctr_at(w.ctr, C_KQ0 + k) = 0u; }
+  *ctr_at(w.ctr, C_WAVES) = wave + 1u;
+}
+
 template<class J>
 __global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
+  if(blockIdx.x == 0 && threadIdx.x == 0) { wave_begin(w); }
   const uint32_t cur = wave_of(w) & 1u;
   const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_ACT0 + cur);
   ExtendQueue<J> q{jobs, w, w.sorted ? w.sort_val[1] : w.active[cur], LaneScene<J>(jobs), 0u,
@@ -674,7 +712,7 @@ __global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
 //        ray escapes, and L and w depend on the direction alone, so it is an
 //        any-hit query with its contribution computed here;
 //   nb   the BSDF strategy towards an area light: closest hit, L and the MIS
-//        weight once the hit is known (wf_neeb).
+//        weight once the hit is known (NeebQueue).
 struct NeeEntries {
   bool sh, sh2, nb;
   float4 sh_o, sh_d, sh_c, sh2_o, sh2_d, sh2_c, nb_o, nb_d, nb_f;
@@ -759,15 +797,24 @@ __device__ __forceinline__ void push_entries(WfDev& w, uint32_t slot, const NeeE
   }
 }
 
-#ifdef DORT_SHADE_MAXNREG
-#define DORT_SHADE_REGS __maxnreg__(DORT_SHADE_MAXNREG)
-#else
-#define DORT_SHADE_REGS
-#endif
+// Register cap of the shade stage: four blocks of 128 threads per SM for the
+// triangle-scene instantiation (without it the loop's call takes it to 131
+// registers and three blocks: 35.0 against 34.2 ms on the 16-spp 1080p frame);
+// the general one needs 198.
+#define DORT_SHADE_REGS __maxnreg__(J::kGeneral ? 200 : 128)
+
+// The loop of a frame's graph (`on` = 0 outside a graph).  shade passes C_MORE
+// on to it: the call costs the trace stages registers that they need.
+struct WfLoop {
+  cudaGraphConditionalHandle handle;
+  uint32_t on;
+};
 
 template<class J>
-__global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w) {
-  const uint32_t cur = wave_of(w) & 1u;
+__global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
+  if(loop.on && blockIdx.x == 0 && threadIdx.x == 0) {
+    cudaGraphSetConditional(loop.handle, *ctr_at(w.ctr, C_MORE));
+  }
   uint32_t qn[kShadeQueues];
   uint32_t n = 0;
 #pragma unroll
@@ -1029,8 +1076,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return __any_sync(0xffffffffu, done != 0);
 }
 
+// The shadow queue of a wave.
 template<class J, bool STAGED>
-__global__ void DORT_TRACE_REGS wf_shadow(J jobs, WfDev w) {
+__device__ __forceinline__ void trace_shadow(J& jobs, WfDev& w) {
   const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_SHADOW);
   const uint32_t lane = threadIdx.x & 31u;
   if(STAGED && blockDim.x <= 32 * kTmaWarps) {
@@ -1138,44 +1186,21 @@ struct NeebQueue {
   }
 };
 
-template<class J>
-__global__ void DORT_TRACE_REGS wf_neeb(J jobs, WfDev w) {
-  const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_NEEB);
-  NeebQueue<J> q{jobs, w, LaneScene<J>(jobs)};
-  trace_queue<false, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_NB));
-}
+// The direct lighting of a wave: its shadow queue, its BSDF-strategy queue,
+// and the end of the wave (`parts`; one launch does all three, the stage
+// timing one after the other).  One kernel, so that a warp goes on with the
+// second queue while others finish the first.
+enum : uint32_t { LIGHT_SHADOW = 1, LIGHT_NEEB = 2, LIGHT_END = 4, LIGHT_ALL = 7 };
 
-// Single thread: account the wave, retire its queues, decide whether to loop.
-__device__ __forceinline__ bool wf_end_wave(WfDev& w) {
-  uint32_t wave = *ctr_at(w.ctr, C_WAVES);
-  uint32_t cur = wave & 1u;
-  uint32_t a = *ctr_at(w.ctr, C_ACT0 + cur), s = *ctr_at(w.ctr, C_SHADOW), b = *ctr_at(w.ctr, C_NEEB);
-  unsigned long long* rays = reinterpret_cast<unsigned long long*>(ctr_at(w.ctr, C_RAYS_LO));
-  *rays += (unsigned long long)a + s + b;
-  // this wave's active queue stays for the next regen; the lists this wave's
-  // regen read are consumed
-  *ctr_at(w.ctr, C_ACT0 + (cur ^ 1u)) = 0u;
-  *ctr_at(w.ctr, C_FIN0 + cur) = 0u;
-  *ctr_at(w.ctr, C_SHADOW) = 0u;
-  *ctr_at(w.ctr, C_NEEB) = 0u;
-  *ctr_at(w.ctr, C_F_EXT) = 0u;
-  *ctr_at(w.ctr, C_F_SHADE) = 0u;
-  *ctr_at(w.ctr, C_F_SH) = 0u;
-  *ctr_at(w.ctr, C_F_NB) = 0u;
-  for(uint32_t k = 0; k < kShadeQueues; ++k) { *ctr_at(w.ctr, C_KQ0 + k) = 0u; }
-  *ctr_at(w.ctr, C_WAVES) = wave + 1u;
-  uint64_t next = *reinterpret_cast<uint64_t*>(ctr_at(w.ctr, C_NEXT_LO));
-  bool more = *ctr_at(w.ctr, C_LIVE) > 0u || next < w.total_samples;
-  if(more && wave + 1u >= w.max_waves) {
-    // bounded: a frame never loops forever; the host reports the error
-    *ctr_at(w.ctr, C_ERROR) = 1u;
-    more = false;
+template<class J, bool STAGED>
+__global__ void DORT_TRACE_REGS wf_light(J jobs, WfDev w, uint32_t parts) {
+  if((parts & LIGHT_END) && blockIdx.x == 0 && threadIdx.x == 0) { wave_end(w); }
+  if(parts & LIGHT_SHADOW) { trace_shadow<J, STAGED>(jobs, w); }
+  if(parts & LIGHT_NEEB) {
+    const uint32_t n = *(volatile uint32_t*)ctr_at(w.ctr, C_NEEB);
+    NeebQueue<J> q{jobs, w, LaneScene<J>(jobs)};
+    trace_queue<false, false, kTraceTest<J::kGeneral>>(q, n, ctr_at(w.ctr, C_F_NB));
   }
-  return more;
-}
-
-__global__ void wf_control(WfDev w, cudaGraphConditionalHandle handle) {
-  cudaGraphSetConditional(handle, wf_end_wave(w) ? 1u : 0u);
 }
 
 __global__ void wf_resolve(WfDev w, uint32_t npix, float* __restrict__ out) {
@@ -1345,8 +1370,8 @@ static int grid_for(const void* kernel, int block, size_t shared = 0) {
 // that a kernel's registers do not allow (threads x registers above the
 // SM's register file) is lowered to the kernel's limit, a multiple of 32.
 struct WfGrids {
-  int regen, ext, sha, shw, nb;
-  int b_ext, b_sha, b_shw, b_nb;
+  int regen, ext, sha, light;
+  int b_ext, b_sha, b_light;
 };
 
 static int fit_block(const void* kernel, int block) {
@@ -1363,18 +1388,15 @@ static WfGrids wf_grids(const WfTuning& tn) {
   WfGrids g;
   const void* ext = reinterpret_cast<const void*>(&wf_extend<J>);
   const void* sha = reinterpret_cast<const void*>(&wf_shade<J>);
-  const void* shw = tn.stage_queues ? reinterpret_cast<const void*>(&wf_shadow<J, true>)
-                                    : reinterpret_cast<const void*>(&wf_shadow<J, false>);
-  const void* nb = reinterpret_cast<const void*>(&wf_neeb<J>);
+  const void* light = tn.stage_queues ? reinterpret_cast<const void*>(&wf_light<J, true>)
+                                      : reinterpret_cast<const void*>(&wf_light<J, false>);
   g.b_ext = fit_block(ext, int(tn.trace_block));
   g.b_sha = fit_block(sha, int(tn.shade_block));
-  g.b_shw = fit_block(shw, int(tn.trace_block));
-  g.b_nb = fit_block(nb, int(tn.trace_block));
+  g.b_light = fit_block(light, int(tn.trace_block));
   g.regen = grid_for(reinterpret_cast<const void*>(&wf_regen<J>), int(kRegenBlock));
   g.ext = grid_for(ext, g.b_ext, WarpBuffer<2>::bytes(g.b_ext));
   g.sha = grid_for(sha, g.b_sha);
-  g.shw = grid_for(shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw));
-  g.nb = grid_for(nb, g.b_nb);
+  g.light = grid_for(light, g.b_light, WarpBuffer<1>::bytes(g.b_light));
   return g;
 }
 
@@ -1389,7 +1411,7 @@ static void wf_sort(const J& jobs, WfDev& dev, const WfGrids& g, cudaStream_t st
 }
 
 // The extension stage (with the ray sort and the classification that go
-// with it) and the shadow stage in the variants the tuning selects.
+// with it) and the light stage in the variants the tuning selects.
 template<class J>
 static void wf_launch_extend(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
                              cudaStream_t st) {
@@ -1399,23 +1421,23 @@ static void wf_launch_extend(const J& jobs, WfDev& dev, const WfTuning& tn, cons
 }
 
 template<class J>
-static void wf_launch_shadow(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
-                             cudaStream_t st) {
+static void wf_launch_light(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
+                            uint32_t parts, cudaStream_t st) {
+  const size_t shared = WarpBuffer<1>::bytes(g.b_light);
   if(tn.stage_queues) {
-    wf_shadow<J, true><<<g.shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw), st>>>(jobs, dev);
+    wf_light<J, true><<<g.light, g.b_light, shared, st>>>(jobs, dev, parts);
   } else {
-    wf_shadow<J, false><<<g.shw, g.b_shw, WarpBuffer<1>::bytes(g.b_shw), st>>>(jobs, dev);
+    wf_light<J, false><<<g.light, g.b_light, shared, st>>>(jobs, dev, parts);
   }
 }
 
 template<class J>
 static void wf_launch_wave(const J& jobs, WfDev& dev, const WfTuning& tn, const WfGrids& g,
-                           cudaStream_t st) {
+                           WfLoop loop, cudaStream_t st) {
   wf_regen<J><<<g.regen, kRegenBlock, 0, st>>>(jobs, dev);
   wf_launch_extend<J>(jobs, dev, tn, g, st);
-  wf_shade<J><<<g.sha, g.b_sha, 0, st>>>(jobs, dev);
-  wf_launch_shadow<J>(jobs, dev, tn, g, st);
-  wf_neeb<J><<<g.nb, g.b_nb, 0, st>>>(jobs, dev);
+  wf_shade<J><<<g.sha, g.b_sha, 0, st>>>(jobs, dev, loop);
+  wf_launch_light<J>(jobs, dev, tn, g, LIGHT_ALL, st);
 }
 
 template<class J>
@@ -1442,8 +1464,7 @@ static int wf_build_graph(Wavefront* wf, const J& jobs, const WfTuning& tn) {
   wf->dev.sorted = tn.sort;
   DG_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal));
-  wf_launch_wave<J>(jobs, wf->dev, tn, g, st);
-  wf_control<<<1, 1, 0, st>>>(wf->dev, handle);
+  wf_launch_wave<J>(jobs, wf->dev, tn, g, WfLoop{handle, 1u}, st);
   cudaGraph_t captured = nullptr;
   cudaError_t ce = cudaStreamEndCapture(st, &captured);
   if(ce != cudaSuccess) {
@@ -1597,10 +1618,6 @@ int wavefront_adjoint_counters(dort_scene* s, uint64_t* rays, uint32_t* waves, u
 
 // The same frame as wavefront_render, run wave by wave from the host without
 // the graph, with CUDA events around every stage; for measurement only.
-__global__ void wf_control_host(WfDev w, uint32_t* more_flag) {
-  *more_flag = wf_end_wave(w) ? 1u : 0u;
-}
-
 template<bool G>
 static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, float* d_out,
                          cudaStream_t st, double ms[6], double stage_rays[3]) {
@@ -1637,15 +1654,16 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
     // the sort counts as part of the extension stage
     wf_launch_extend<SingleJob<G>>(jobs, wf->dev, tn, g, st);
     cudaEventRecord(ev[2], st);
-    wf_shade<SingleJob<G>><<<g.sha, g.b_sha, 0, st>>>(jobs, wf->dev);
+    wf_shade<SingleJob<G>><<<g.sha, g.b_sha, 0, st>>>(jobs, wf->dev, WfLoop{0, 0u});
     cudaEventRecord(ev[3], st);
-    wf_launch_shadow<SingleJob<G>>(jobs, wf->dev, tn, g, st);
+    wf_launch_light<SingleJob<G>>(jobs, wf->dev, tn, g, LIGHT_SHADOW, st);
     cudaEventRecord(ev[4], st);
-    wf_neeb<SingleJob<G>><<<g.nb, g.b_nb, 0, st>>>(jobs, wf->dev);
+    wf_launch_light<SingleJob<G>>(jobs, wf->dev, tn, g, LIGHT_NEEB | LIGHT_END, st);
     cudaEventRecord(ev[5], st);
     cudaMemcpy2DAsync(more + 1, sizeof(uint32_t), wf->dev.ctr, kCtrStride * sizeof(uint32_t),
                       sizeof(uint32_t), C_NEEB + 1, cudaMemcpyDeviceToHost, st);
-    wf_control_host<<<1, 1, 0, st>>>(wf->dev, more);
+    cudaMemcpyAsync(more, ctr_at(wf->dev.ctr, C_MORE), sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                    st);
     ok = cudaStreamSynchronize(st) == cudaSuccess;
     for(int k = 0; ok && k < 5; ++k) {
       float t = 0.f;
