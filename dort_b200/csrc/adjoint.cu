@@ -54,6 +54,7 @@ int launch_render(dort_scene* s, const PtParams& pp, float* d_out, cudaStream_t 
 #endif
 
 struct AdjointTape {
+  static constexpr int kCalls = 0;
   V3 L;          // sample value from pass 1
   V3 acc;        // terms seen so far
   V3 adj;        // dLoss/dI(pixel) / spp
@@ -94,6 +95,7 @@ struct AdjointTape {
 
 // Terms of one sample in a per-thread log (adjoint.cuh's entries).
 struct AdjointLog {
+  static constexpr int kCalls = 0;
   float4 ev[kAdjLog];
   uint32_t n;
   bool overflow;

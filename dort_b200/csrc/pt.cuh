@@ -385,9 +385,8 @@ DG_HD float bsdf_pdf(const DevMaterial& m, const Frame& fr, V3 wi, V3 wo, uint32
 
 // The analytic shapes (a short list, each tested in its own space against the
 // closest t so far).
-template<bool ANY_HIT>
-DG_HD Hit trace_shapes(const PtScene& sc, V3 o, float t_min, V3 d,
-                                                  float t_max, Hit h) {
+template<bool ANY_HIT, class S>
+DG_HD Hit trace_shapes(const S& sc, V3 o, float t_min, V3 d, float t_max, Hit h) {
   float best = h.prim == kMiss ? t_max : h.t;
   for(uint32_t k = 0; k < sc.shape_count; ++k) {
     const DevShape& s = sc.shapes[k];
@@ -406,16 +405,44 @@ DG_HD Hit trace_shapes(const PtScene& sc, V3 o, float t_min, V3 d,
   return h;
 }
 
+// What a ray query needs of a scene.
+struct QueryScene {
+  TraceScene trace;
+  const DevShape* shapes;
+  uint32_t shape_count, shape_base;
+};
+
 // Scene::intersect / intersect_p (scene.cpp:8-18) over the flat scene: the
 // triangle BVH, then the analytic shapes.  A shape hit has prim = shape_base +
 // its index and b1 = the cube face.
-template<bool ANY_HIT, bool G>
-DG_HD Hit scene_trace(const PtScene& sc, V3 o, float t_min, V3 d, float t_max) {
+template<bool ANY_HIT, bool G, class S>
+DG_HD Hit scene_trace(const S& sc, V3 o, float t_min, V3 d, float t_max) {
   // the general instantiation also serves scenes built watertight
   Hit h = trace_ray<ANY_HIT, false, G ? kTriByScene : kTriMt>(sc.trace, o.x, o.y, o.z, t_min,
                                                              d.x, d.y, d.z, t_max);
   if(!G || sc.shape_count == 0 || (ANY_HIT && h.prim != kMiss)) { return h; }
   return trace_shapes<ANY_HIT>(sc, o, t_min, d, t_max, h);
+}
+
+// The ray queries of the whole-path kernel, out of line: a path's seven
+// query sites hold one copy of the traversal (see pt_megakernel).  Its values
+// pass through memory or loop variables either way, so the call changes no
+// rounding.  kCalls numbers the kernel (a copy for each: ptxas 12.9 does not
+// get through a function that two of these kernels share); 0: inline.
+template<bool ANY_HIT, bool G, int kCalls>
+__host__ __device__ __noinline__ Hit scene_trace_call(QueryScene sc, V3 o, float t_min, V3 d,
+                                                      float t_max) {
+  return scene_trace<ANY_HIT, G>(sc, o, t_min, d, t_max);
+}
+template<bool ANY_HIT, bool G, int kCalls>
+DG_HD Hit path_trace(const PtScene& sc, V3 o, float t_min, V3 d, float t_max) {
+#ifdef __CUDA_ARCH__
+  if constexpr(kCalls != 0) {
+    return scene_trace_call<ANY_HIT, G, kCalls>(
+        QueryScene{sc.trace, sc.shapes, sc.shape_count, sc.shape_base}, o, t_min, d, t_max);
+  }
+#endif
+  return scene_trace<ANY_HIT, G>(sc, o, t_min, d, t_max);
 }
 
 // Material index of a hit primitive.
@@ -753,12 +780,16 @@ DG_HD LightSample light_sample(const PtScene& sc, const DevLight& l, V3 pivot, f
 //   vertex(tri, material)                a scattering vertex starts; every
 //                                        later term is linear in its BSDF
 //   direct(light tri or kMiss, c)        adds c (a direct-lighting term)
-struct NoTape {
+// kCalls: the path's ray queries (path_trace).
+template<int kKernel>
+struct NoTapeOf {
+  static constexpr int kCalls = kKernel;
   DG_HD void emission(uint32_t, V3, V3) {}
   DG_HD void background(V3) {}
   DG_HD void vertex(uint32_t, const DevMaterial&) {}
   DG_HD void direct(uint32_t, V3) {}
 };
+using NoTape = NoTapeOf<0>;
 
 struct PathResult {
   V3 L;
@@ -817,7 +848,7 @@ DG_HD void camera_ray(const PtParams& pp, uint32_t pixel, uint32_t sample, float
 }
 
 // Direct lighting from one light (estimate_direct, path_renderer.cpp:135-206).
-template<bool G>
+template<bool G, int kCalls>
 DG_HD V3 estimate_direct(const PtScene& sc, const PtParams& pp, uint32_t li,
                          const SurfaceHit& g, const DevMaterial& m, V3 wo,
                          float u_bsdf, float v_bsdf, float c_bsdf, float u_l, float v_l,
@@ -834,8 +865,8 @@ DG_HD V3 estimate_direct(const PtScene& sc, const PtParams& pp, uint32_t li,
       // A background light counts only if the ray escapes, so whether anything
       // is hit is all that matters: an any-hit query gives the same answer.
       bool area = light_is_area(l);
-      Hit h = area ? scene_trace<false, G>(sc, g.p, g.eps, bs.w, INFINITY)
-                   : scene_trace<true, G>(sc, g.p, g.eps, bs.w, INFINITY);
+      Hit h = area ? path_trace<false, G, kCalls>(sc, g.p, g.eps, bs.w, INFINITY)
+                   : path_trace<true, G, kCalls>(sc, g.p, g.eps, bs.w, INFINITY);
       rays += 1;
       V3 L = v3(0.f, 0.f, 0.f);
       if(area) {
@@ -858,7 +889,7 @@ DG_HD V3 estimate_direct(const PtScene& sc, const PtParams& pp, uint32_t li,
     if(!(ls.pdf == 0.f || is_black(ls.L))) {
       V3 f = bsdf_eval<G>(m, g.frame, ls.wi, wo, req);
       if(!is_black(f)) {
-        Hit h = scene_trace<true, G>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
+        Hit h = path_trace<true, G, kCalls>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
         rays += 1;
         if(h.prim == kMiss) {
           float w = 1.f;
@@ -874,97 +905,128 @@ DG_HD V3 estimate_direct(const PtScene& sc, const PtParams& pp, uint32_t li,
   return sum;
 }
 
-// PathRenderer::sample (path_renderer.cpp:23-111) for one film position.
+// One path of PathRenderer::sample (path_renderer.cpp:23-111).
+struct PathState {
+  uint32_t pixel, sample;
+  V3 o, d;
+  float tmin;
+  V3 sum, thr;
+  uint32_t bounces;
+  bool last_delta;
+  uint32_t rays;       // closest-hit + shadow rays traced
+};
+
+// Starts the path of sample `sample` of `pixel` at film position (fx, fy).
+template<bool G>
+DG_HD void path_start(PathState& p, const PtParams& pp, uint32_t pixel, uint32_t sample, float fx,
+                      float fy) {
+  p.pixel = pixel;
+  p.sample = sample;
+  camera_ray<G>(pp, pixel, sample, fx, fy, p.o, p.d);
+  p.tmin = 0.f;
+  p.sum = v3(0.f, 0.f, 0.f);
+  p.thr = v3(1.f, 1.f, 1.f);
+  p.bounces = 0;
+  p.last_delta = false;
+  p.rays = 0;
+}
+
+// The path's next ray and vertex; true when the path ends (its value is
+// p.sum: the importance / ray pdf of the cameras is 1).
+template<class Tape, bool G>
+DG_HD bool path_step(PathState& p, const PtScene& sc, const PtParams& pp, Tape& tape) {
+  constexpr int kCalls = Tape::kCalls;
+  V3 &o = p.o, &d = p.d, &sum = p.sum, &thr = p.thr;
+  float& tmin = p.tmin;
+  uint32_t& bounces = p.bounces;
+  bool& last_delta = p.last_delta;
+  const uint32_t req_nd = F_ALL & ~F_DELTA;
+  Hit h = path_trace<false, G, kCalls>(sc, o, tmin, d, INFINITY);
+  p.rays += 1;
+  bool hit = h.prim != kMiss;
+  SurfaceHit g;
+  if(hit) { g = surface_at<G>(sc, h, o, d); }
+  if((bounces == 0 || last_delta) && bounces >= pp.min_depth && bounces <= pp.max_depth) {
+    if(hit) {
+      if(g.light) {
+        const DevLight& l = sc.lights[g.light - 1];
+        V3 Le = area_eval_radiance(sc, l, g.p, g.n, o);
+        tape.emission(g.tri, thr, Le);
+        sum = sum + thr * Le;
+      }
+    } else {
+      for(uint32_t k = 0; k < sc.bg_count; ++k) {
+        V3 c = thr * background_radiance(sc, sc.lights[sc.bg_light[k]], d);
+        tape.background(c);
+        sum = sum + c;
+      }
+    }
+  }
+  bounces += 1;
+  if(!hit || bounces > pp.max_depth) { return true; }
+
+  V3 wo = normalize(-d);
+  DevMaterial m = material_at(sc, g);
+  uint32_t blk = bounce_block(bounces);
+  Rand4 r0 = rand4(pp.seed, p.pixel, p.sample, blk);
+  Rand4 r1 = rand4(pp.seed, p.pixel, p.sample, blk + 1);
+  Rand4 r2 = rand4(pp.seed, p.pixel, p.sample, blk + 2);
+
+  tape.vertex(g.tri, m);
+  if(bounces >= pp.min_depth && bxdf_matches(m.bxdf_flags, req_nd)) {
+    // sample_direct_lighting (path_renderer.cpp:113-132)
+    if(pp.sample_all_lights) {
+      for(uint32_t li = 0; li < sc.light_count; ++li) {
+        uint32_t b2 = all_lights_block(bounces, li, sc.light_count);
+        Rand4 a = rand4(pp.seed, p.pixel, p.sample, b2);
+        Rand4 b = rand4(pp.seed, p.pixel, p.sample, b2 + 1);
+        const DevLight& l = sc.lights[li];
+        V3 c = estimate_direct<G, kCalls>(sc, pp, li, g, m, wo, a.a, a.b, a.c, b.a, b.b, p.rays) * thr;
+        tape.direct(l.kind == LIGHT_TRI ? l.tri : kMiss, c);
+        sum = sum + c;
+      }
+    } else if(sc.light_count > 0) {
+      uint32_t li = distrib_sample(sc.light_cdf, sc.light_count + 1, r0.a);
+      float lpdf = distrib_pdf(sc.light_cdf, sc.light_count + 1, li);
+      if(lpdf != 0.f) {
+        const DevLight& l = sc.lights[li];
+        V3 e = estimate_direct<G, kCalls>(sc, pp, li, g, m, wo, r0.b, r0.c, r0.d, r1.a, r1.b, p.rays);
+        V3 c = e * (1.f / lpdf) * thr;
+        tape.direct(l.kind == LIGHT_TRI ? l.tri : kMiss, c);
+        sum = sum + c;
+      }
+    }
+  }
+
+  uint32_t req = (pp.only_direct || bounces == pp.max_depth) ? (F_MODES | F_DELTA) : F_ALL;
+  BsdfSample bs = bsdf_sample<G>(m, g.frame, wo, req, r1.c, r1.d, r2.a);
+  if(is_black(bs.f) || bs.pdf == 0.f) { return true; }
+  V3 contrib = bs.f * (fabsf(dot(bs.w, g.n)) / bs.pdf);
+  last_delta = (bs.flags & F_DELTA) != 0;
+  thr = thr * contrib;
+  if(bounces == pp.max_depth && !last_delta) {
+    return true;
+  } else if(bounces >= 2 && bounces > pp.min_depth && pp.roulette) {
+    float survive = clampf(average(contrib), 0.1f, 0.99f);
+    if(r2.b > survive) { return true; }
+    thr = thr * (1.f / survive);
+  }
+  o = g.p;
+  d = bs.w;
+  tmin = g.eps;
+  return false;
+}
+
+// One whole sample at one film position.
 template<class Tape, bool G>
 DG_HD PathResult pt_sample(const PtScene& sc, const PtParams& pp, uint32_t pixel,
                            uint32_t sample, float fx, float fy, Tape& tape) {
+  PathState p;
+  path_start<G>(p, pp, pixel, sample, fx, fy);
+  while(!path_step<Tape, G>(p, sc, pp, tape)) {}
   PathResult res;
-  res.rays = 0;
-  V3 o, d;
-  camera_ray<G>(pp, pixel, sample, fx, fy, o, d);
-  float tmin = 0.f;
-  V3 sum = v3(0.f, 0.f, 0.f);
-  V3 thr = v3(1.f, 1.f, 1.f);
-  uint32_t bounces = 0;
-  bool last_delta = false;
-  const uint32_t req_nd = F_ALL & ~F_DELTA;
-  for(;;) {
-    Hit h = scene_trace<false, G>(sc, o, tmin, d, INFINITY);
-    res.rays += 1;
-    bool hit = h.prim != kMiss;
-    SurfaceHit g;
-    if(hit) { g = surface_at<G>(sc, h, o, d); }
-    if((bounces == 0 || last_delta) && bounces >= pp.min_depth && bounces <= pp.max_depth) {
-      if(hit) {
-        if(g.light) {
-          const DevLight& l = sc.lights[g.light - 1];
-          V3 Le = area_eval_radiance(sc, l, g.p, g.n, o);
-          tape.emission(g.tri, thr, Le);
-          sum = sum + thr * Le;
-        }
-      } else {
-        for(uint32_t k = 0; k < sc.bg_count; ++k) {
-          V3 c = thr * background_radiance(sc, sc.lights[sc.bg_light[k]], d);
-          tape.background(c);
-          sum = sum + c;
-        }
-      }
-    }
-    bounces += 1;
-    if(!hit || bounces > pp.max_depth) { break; }
-
-    V3 wo = normalize(-d);
-    DevMaterial m = material_at(sc, g);
-    uint32_t blk = bounce_block(bounces);
-    Rand4 r0 = rand4(pp.seed, pixel, sample, blk);
-    Rand4 r1 = rand4(pp.seed, pixel, sample, blk + 1);
-    Rand4 r2 = rand4(pp.seed, pixel, sample, blk + 2);
-
-    tape.vertex(g.tri, m);
-    if(bounces >= pp.min_depth && bxdf_matches(m.bxdf_flags, req_nd)) {
-      // sample_direct_lighting (path_renderer.cpp:113-132)
-      if(pp.sample_all_lights) {
-        for(uint32_t li = 0; li < sc.light_count; ++li) {
-          uint32_t b2 = all_lights_block(bounces, li, sc.light_count);
-          Rand4 a = rand4(pp.seed, pixel, sample, b2);
-          Rand4 b = rand4(pp.seed, pixel, sample, b2 + 1);
-          const DevLight& l = sc.lights[li];
-          V3 c = estimate_direct<G>(sc, pp, li, g, m, wo, a.a, a.b, a.c, b.a, b.b, res.rays) * thr;
-          tape.direct(l.kind == LIGHT_TRI ? l.tri : kMiss, c);
-          sum = sum + c;
-        }
-      } else if(sc.light_count > 0) {
-        uint32_t li = distrib_sample(sc.light_cdf, sc.light_count + 1, r0.a);
-        float lpdf = distrib_pdf(sc.light_cdf, sc.light_count + 1, li);
-        if(lpdf != 0.f) {
-          const DevLight& l = sc.lights[li];
-          V3 e = estimate_direct<G>(sc, pp, li, g, m, wo, r0.b, r0.c, r0.d, r1.a, r1.b, res.rays);
-          V3 c = e * (1.f / lpdf) * thr;
-          tape.direct(l.kind == LIGHT_TRI ? l.tri : kMiss, c);
-          sum = sum + c;
-        }
-      }
-    }
-
-    uint32_t req = (pp.only_direct || bounces == pp.max_depth) ? (F_MODES | F_DELTA) : F_ALL;
-    BsdfSample bs = bsdf_sample<G>(m, g.frame, wo, req, r1.c, r1.d, r2.a);
-    if(is_black(bs.f) || bs.pdf == 0.f) { break; }
-    V3 contrib = bs.f * (fabsf(dot(bs.w, g.n)) / bs.pdf);
-    last_delta = (bs.flags & F_DELTA) != 0;
-    thr = thr * contrib;
-    if(bounces == pp.max_depth && !last_delta) {
-      break;
-    } else if(bounces >= 2 && bounces > pp.min_depth && pp.roulette) {
-      float survive = clampf(average(contrib), 0.1f, 0.99f);
-      if(r2.b > survive) { break; }
-      thr = thr * (1.f / survive);
-    }
-    o = g.p;
-    d = bs.w;
-    tmin = g.eps;
-  }
-  // importance / ray_pdf of the pinhole camera is 1
-  res.L = sum;
+  res.L = p.sum;
+  res.rays = p.rays;
   return res;
 }
 

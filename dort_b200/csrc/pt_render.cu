@@ -43,12 +43,15 @@ DG_HD bool keep_sample(V3 L) {
          L.z >= 0.f;
 }
 
-// Resident blocks per SM the register allocation must allow: 5 (96
-// registers) against the block size alone (168 registers): the Cornell
-// workload 557 against 468 M samples/s, the 1080p frame 286.6 against 282.1
-// M (6 blocks: 573 and 273.4 M).
+// Resident blocks per SM the register allocation must allow: 6 (80 registers).
+// What bounds the kernel is instruction fetch (ncu, the general instantiation
+// with its queries inlined: 32 of 37 cycles per issue without an instruction),
+// so its ray queries are calls (path_trace), and more warps hide the rest: a
+// 200x150 frame of the general scene at 32 spp took 7.36 ms with the queries
+// inlined and 5 blocks, 5.86 with calls, 5.57 with calls and 6 blocks (7: 5.61,
+// 8: 5.44, but 3.00 against 2.92 ms on the Cornell box).
 #ifndef DORT_PT_MIN_BLOCKS
-#define DORT_PT_MIN_BLOCKS 5
+#define DORT_PT_MIN_BLOCKS 6
 #endif
 // 0: the block size alone (the compiler picks the registers)
 #if DORT_PT_MIN_BLOCKS > 0
@@ -57,7 +60,14 @@ DG_HD bool keep_sample(V3 L) {
 #define DORT_PT_BOUNDS __launch_bounds__(kPtBlock)
 #endif
 
-template<bool G>
+// Samples per thread from which a thread whose path has ended starts its next
+// sample while the warp's other paths go on (kRegenerate), instead of waiting
+// for them: at 32 spp the Cornell box (4 samples per thread) 2.92 -> 2.62 ms, a
+// 300x300 frame of the general scene at 128 spp (22) 65.3 -> 54.0 ms; with 2
+// samples per thread the flags cost more than that gives (5.60 -> 5.74 ms).
+constexpr uint32_t kRegenerateFrom = 4;
+
+template<bool G, bool kRegenerate>
 __global__ void DORT_PT_BOUNDS
 pt_megakernel(PtScene sc, PtParams pp, uint32_t slices, uint32_t spp_per_slice,
               uint32_t per_slice, float4* __restrict__ partial,
@@ -79,17 +89,39 @@ pt_megakernel(PtScene sc, PtParams pp, uint32_t slices, uint32_t spp_per_slice,
       uint32_t pixel = y * pp.width + x;
       uint32_t s0 = slice * spp_per_slice;
       uint32_t s1 = min(pp.spp, s0 + spp_per_slice);
-      NoTape tape;
-      for(uint32_t s = s0; s < s1; ++s) {
-        float fx, fy;
-        film_pos(pp, pixel, x, y, s, fx, fy);
-        PathResult r = pt_sample<NoTape, G>(sc, pp, pixel, s, fx, fy, tape);
-        rays += r.rays;
-        if(keep_sample(r.L)) {
-          acc.x += r.L.x;
-          acc.y += r.L.y;
-          acc.z += r.L.z;
+      using Tape = NoTapeOf<kRegenerate ? 2 : 1>;
+      Tape tape;
+      auto keep = [&](V3 L) {
+        if(keep_sample(L)) {
+          acc.x += L.x;
+          acc.y += L.y;
+          acc.z += L.z;
           acc.w += 1.f;
+        }
+      };
+      if constexpr(kRegenerate) {
+        PathState p;
+        bool fresh = true;
+        for(uint32_t s = s0; s < s1;) {
+          if(fresh) {
+            float fx, fy;
+            film_pos(pp, pixel, x, y, s, fx, fy);
+            path_start<G>(p, pp, pixel, s, fx, fy);
+          }
+          fresh = path_step<Tape, G>(p, sc, pp, tape);
+          if(fresh) {
+            rays += p.rays;
+            keep(p.sum);
+            ++s;
+          }
+        }
+      } else {
+        for(uint32_t s = s0; s < s1; ++s) {
+          float fx, fy;
+          film_pos(pp, pixel, x, y, s, fx, fy);
+          PathResult r = pt_sample<Tape, G>(sc, pp, pixel, s, fx, fy, tape);
+          rays += r.rays;
+          keep(r.L);
         }
       }
       partial[size_t(slice) * npix + pixel] = acc;
@@ -99,11 +131,6 @@ pt_megakernel(PtScene sc, PtParams pp, uint32_t slices, uint32_t spp_per_slice,
   for(int o = 16; o > 0; o >>= 1) { rays += __shfl_down_sync(0xffffffffu, rays, o); }
   if((threadIdx.x & 31) == 0 && rays) { atomicAdd(ray_count, (unsigned long long)rays); }
 }
-
-template __global__ void pt_megakernel<false>(PtScene, PtParams, uint32_t, uint32_t, uint32_t,
-                                               float4*, unsigned long long*);
-template __global__ void pt_megakernel<true>(PtScene, PtParams, uint32_t, uint32_t, uint32_t,
-                                              float4*, unsigned long long*);
 
 __global__ void pt_resolve(const float4* __restrict__ partial, uint32_t slices, uint32_t npix,
                            float* __restrict__ out_rgb, unsigned long long* __restrict__ kept) {
@@ -259,6 +286,32 @@ int render_image_buffer(dort_scene* s, size_t bytes, float** out) {
   return DORT_OK;
 }
 
+// The megakernel over `plan`'s threads and the resolve of its partial sums
+// (slices x pixels float4) into d_out; d_counters[0] += rays, [1] += samples
+// kept.
+int launch_megakernel(const PtScene& sc, const PtParams& pp, const MegaPlan& plan,
+                      float4* partial, float* d_out, unsigned long long* d_counters,
+                      cudaStream_t st) {
+  const uint32_t npix = pp.width * pp.height;
+  const uint64_t threads = uint64_t(plan.slices) * plan.per_slice;
+  const uint32_t blocks = uint32_t((threads + kPtBlock - 1) / kPtBlock);
+  auto launch = [&](auto kernel) {
+    kernel<<<blocks, kPtBlock, 0, st>>>(sc, pp, plan.slices, plan.per, plan.per_slice, partial,
+                                        d_counters);
+  };
+  const bool general = scene_needs_general(sc, pp);
+  if(plan.per >= kRegenerateFrom) {
+    if(general) { launch(pt_megakernel<true, true>); } else { launch(pt_megakernel<false, true>); }
+  } else {
+    if(general) { launch(pt_megakernel<true, false>); } else { launch(pt_megakernel<false, false>); }
+  }
+  DG_CUDA(cudaGetLastError());
+  pt_resolve<<<(npix + 255) / 256, 256, 0, st>>>(partial, plan.slices, npix, d_out,
+                                                 d_counters + 1);
+  DG_CUDA(cudaGetLastError());
+  return DORT_OK;
+}
+
 int launch_render(dort_scene* s, const PtParams& pp, float* d_out, cudaStream_t st,
                   unsigned long long* d_counters) {
   int drc = require_scene_device(s);
@@ -275,25 +328,11 @@ int launch_render(dort_scene* s, const PtParams& pp, float* d_out, cudaStream_t 
   if(megakernel_plan(s->device, dev, sms, pp.width, pp.height, pp.spp, 0, &plan) != 0) {
     return fail(DORT_ERR_INVALID, plan.why);
   }
-  const uint32_t slices = plan.slices, per = plan.per, per_slice = plan.per_slice;
-  size_t partial_bytes = size_t(slices) * npix * sizeof(float4);
+  size_t partial_bytes = size_t(plan.slices) * npix * sizeof(float4);
   void* scratch = nullptr;
   int rc = render_scratch(s, partial_bytes, &scratch);
   if(rc != DORT_OK) { return rc; }
-  float4* partial = static_cast<float4*>(scratch);
-  uint64_t threads = uint64_t(slices) * per_slice;
-  uint32_t blocks = uint32_t((threads + kPtBlock - 1) / kPtBlock);
-  if(scene_needs_general(s->pt, pp)) {
-    pt_megakernel<true><<<blocks, kPtBlock, 0, st>>>(s->pt, pp, slices, per, per_slice, partial,
-                                                     d_counters);
-  } else {
-    pt_megakernel<false><<<blocks, kPtBlock, 0, st>>>(s->pt, pp, slices, per, per_slice, partial,
-                                                      d_counters);
-  }
-  DG_CUDA(cudaGetLastError());
-  pt_resolve<<<(npix + 255) / 256, 256, 0, st>>>(partial, slices, npix, d_out, d_counters + 1);
-  DG_CUDA(cudaGetLastError());
-  return DORT_OK;
+  return launch_megakernel(s->pt, pp, plan, static_cast<float4*>(scratch), d_out, d_counters, st);
 }
 
 }  // namespace dort_gpu

@@ -36,13 +36,10 @@
 
 namespace dort_gpu {
 
-// The megakernel (both instantiations) and its resolve step (pt_render.cu).
-template<bool G>
-__global__ void pt_megakernel(PtScene sc, PtParams pp, uint32_t slices, uint32_t spp_per_slice,
-                              uint32_t per_slice, float4* __restrict__ partial,
-                              unsigned long long* __restrict__ ray_count);
-__global__ void pt_resolve(const float4* __restrict__ partial, uint32_t slices, uint32_t npix,
-                           float* __restrict__ out_rgb, unsigned long long* __restrict__ kept);
+// The megakernel and its resolve step (pt_render.cu).
+int launch_megakernel(const PtScene& sc, const PtParams& pp, const MegaPlan& plan,
+                      float4* partial, float* d_out, unsigned long long* d_counters,
+                      cudaStream_t st);
 bool make_params(const dort_render_params* rp, PtParams& pp, std::string& err);
 
 constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;   // 16 MiB per GPU
@@ -108,8 +105,7 @@ extern "C" int dort_gpu_render_device_noalloc(dort_scene* scene,
                      &plan) != 0) {
     return fail(DORT_ERR_INVALID, std::string("dort_gpu_render_device_noalloc: ") + plan.why);
   }
-  const uint32_t slices = plan.slices, per = plan.per, per_slice = plan.per_slice;
-  if(size_t(slices) * npix > kNoAllocMaxPixels) {
+  if(size_t(plan.slices) * npix > kNoAllocMaxPixels) {
     return fail(DORT_ERR_INVALID, "partial sums exceed the no-alloc scratch");
   }
   void* scratch = nullptr;
@@ -120,18 +116,5 @@ extern "C" int dort_gpu_render_device_noalloc(dort_scene* scene,
   unsigned long long* counters = static_cast<unsigned long long*>(scratch);
   float4* partial = reinterpret_cast<float4*>(static_cast<char*>(scratch) + kNoAllocHeader);
   DG_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st));
-  uint64_t threads = uint64_t(slices) * per_slice;
-  const int block = 128;   // the megakernel's launch bound
-  if(scene_needs_general(scene->pt, pp)) {
-    pt_megakernel<true><<<uint32_t((threads + block - 1) / block), block, 0, st>>>(
-        scene->pt, pp, slices, per, per_slice, partial, counters);
-  } else {
-    pt_megakernel<false><<<uint32_t((threads + block - 1) / block), block, 0, st>>>(
-        scene->pt, pp, slices, per, per_slice, partial, counters);
-  }
-  DG_CUDA(cudaGetLastError());
-  pt_resolve<<<uint32_t((npix + 255) / 256), 256, 0, st>>>(partial, slices, uint32_t(npix),
-                                                            d_out_rgb, counters + 1);
-  DG_CUDA(cudaGetLastError());
-  return DORT_OK;
+  return launch_megakernel(scene->pt, pp, plan, partial, d_out_rgb, counters, st);
 } DORT_ABI_CATCH
