@@ -426,6 +426,60 @@ bool validate_mesh(const float* verts, uint32_t vert_count, const uint32_t* tris
   return true;
 }
 
+bool scan_mesh(const float* verts, uint32_t vert_count, const uint32_t* tris, uint32_t tri_count,
+               float lo[3], float hi[3], std::string& err) {
+  struct Part {
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool ok = true;
+  };
+  auto scan = [&](uint32_t begin, uint32_t end, Part& part) {
+    for(uint32_t i = begin; i < end; ++i) {
+      for(int k = 0; k < 3; ++k) {
+        const uint32_t vi = tris[3 * size_t(i) + k];
+        if(vi >= vert_count) { part.ok = false; return; }
+        const float* v = verts + 3 * size_t(vi);
+        for(int a = 0; a < 3; ++a) {
+          // also false for NaN
+          if(!(std::fabs(v[a]) <= 1e15f)) { part.ok = false; return; }
+          part.lo[a] = std::min(part.lo[a], v[a]);
+          part.hi[a] = std::max(part.hi[a], v[a]);
+        }
+      }
+    }
+  };
+  constexpr uint32_t kPerThread = 32768;
+  const uint32_t threads = std::max(1u, std::min({tri_count / kPerThread, 8u,
+                                                  std::thread::hardware_concurrency()}));
+  std::vector<Part> parts(threads);
+  std::vector<std::thread> pool;
+  auto begin_of = [&](uint32_t k) { return uint32_t(uint64_t(tri_count) * k / threads); };
+  uint32_t started = 1;   // part 0 runs here
+  pool.reserve(threads);
+  try {
+    for(; started < threads; ++started) {
+      pool.emplace_back(scan, begin_of(started), begin_of(started + 1), std::ref(parts[started]));
+    }
+  } catch(...) {}         // no more threads: the rest runs here too
+  scan(0, begin_of(1), parts[0]);
+  for(uint32_t k = started; k < threads; ++k) { scan(begin_of(k), begin_of(k + 1), parts[k]); }
+  for(std::thread& t : pool) { t.join(); }
+  for(const Part& part : parts) {
+    // the first fault's message is the one-pass check's
+    if(!part.ok) { return validate_mesh(verts, vert_count, tris, tri_count, err); }
+  }
+  if(tri_count > 0) {
+    for(int a = 0; a < 3; ++a) {
+      lo[a] = INFINITY;
+      hi[a] = -INFINITY;
+      for(const Part& part : parts) {
+        lo[a] = std::min(lo[a], part.lo[a]);
+        hi[a] = std::max(hi[a], part.hi[a]);
+      }
+    }
+  }
+  return true;
+}
+
 bool build_wide_bvh(const float* verts, uint32_t vert_count,
                     const uint32_t* tris, uint32_t tri_count,
                     const BuildOptions& opts, WideBvh& out, std::string& err) {

@@ -135,6 +135,13 @@ double wide_sah_cost(const TraceNode* nodes, size_t node_count);
 bool validate_mesh(const float* verts, uint32_t vert_count, const uint32_t* tris,
                    uint32_t tri_count, std::string& err);
 
+// validate_mesh and the bounds of the vertices that triangles use, in one pass
+// over the mesh on several threads (a 500k-triangle scene spent 8 of its 17 ms
+// of creation on two passes of one thread).  lo / hi are only written for a
+// valid mesh with triangles.
+bool scan_mesh(const float* verts, uint32_t vert_count, const uint32_t* tris, uint32_t tri_count,
+               float lo[3], float hi[3], std::string& err);
+
 // Builds the wide BVH; returns false (with a message) on invalid input.
 bool build_wide_bvh(const float* verts, uint32_t vert_count,
                     const uint32_t* tris, uint32_t tri_count,

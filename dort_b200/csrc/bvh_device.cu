@@ -788,22 +788,53 @@ __global__ void k_emit(const DevBin* __restrict__ nodes, const uint32_t* __restr
   wide_out[qwide[i]] = packed;
 }
 
-// Device buffers of one build, freed together.
+// Shading records by original triangle index (PtScene::shade): the vertices,
+// with the material index and the light index + 1 in the spare words.
+__global__ void k_shade(const float* __restrict__ verts, const uint32_t* __restrict__ tris,
+                        const uint32_t* __restrict__ material, const uint32_t* __restrict__ light,
+                        uint32_t n, float4* __restrict__ shade) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if(t >= n) { return; }
+  const float w[3] = {__uint_as_float(material ? material[t] : 0u),
+                      __uint_as_float(light ? light[t] : 0u), 0.f};
+  for(uint32_t k = 0; k < 3; ++k) {
+    const float* p = verts + 3 * size_t(tris[3 * size_t(t) + k]);
+    shade[3 * size_t(t) + k] = make_float4(p[0], p[1], p[2], w[k]);
+  }
+}
+
+// Device buffers of one build, carved out of a few allocations and freed
+// together.  One allocation per buffer cost a build of 500k triangles 7.4 ms in
+// its 40 cudaFree calls and about as much in cudaMalloc.
 struct Scratch {
-  std::vector<void*> bufs;
+  std::vector<void*> blocks;
+  char* at = nullptr;
+  size_t room = 0;
+  static size_t padded(size_t bytes) { return (std::max<size_t>(bytes, 1) + 255) & ~size_t(255); }
+  // The next buffers take `bytes` (padded) together; they may take more.
+  bool reserve(size_t bytes, std::string& err) {
+    void* p = nullptr;
+    if(dev_alloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      err = "cudaMalloc of " + std::to_string(bytes) + " bytes failed (BVH build)";
+      return false;
+    }
+    blocks.push_back(p);
+    at = static_cast<char*>(p);
+    room = bytes;
+    return true;
+  }
   template<class T>
   T* alloc(size_t count, std::string& err) {
-    void* p = nullptr;
-    if(dev_alloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
-      cudaGetLastError();
-      err = "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes failed (BVH build)";
-      return nullptr;
-    }
-    bufs.push_back(p);
-    return static_cast<T*>(p);
+    const size_t bytes = padded(count * sizeof(T));
+    if(bytes > room && !reserve(bytes, err)) { return nullptr; }
+    char* p = at;
+    at += bytes;
+    room -= bytes;
+    return reinterpret_cast<T*>(p);
   }
   ~Scratch() {
-    for(void* p : bufs) { cudaFree(p); }
+    for(void* p : blocks) { cudaFree(p); }
   }
 };
 
@@ -845,6 +876,12 @@ float decode_ordered(uint32_t u) {
   float f;
   std::memcpy(&f, &b, 4);
   return f;
+}
+
+size_t ploc_bytes(uint32_t n) {
+  const size_t total_nodes = 2 * size_t(n) - 1;
+  return 4 * Scratch::padded(size_t(n) * 8) + 5 * Scratch::padded(size_t(n) * 4) +
+         Scratch::padded(total_nodes * sizeof(DevBin)) + Scratch::padded(total_nodes * 4);
 }
 
 bool build_ploc(Scratch& sc, const DevBin* prim, const uint32_t* bounds, uint32_t n,
@@ -911,13 +948,30 @@ bool build_ploc(Scratch& sc, const DevBin* prim, const uint32_t* bounds, uint32_
   return true;
 }
 
+// The capacities of a binned SAH build of n triangles.
+struct SahSizes {
+  uint32_t tasks;    // open tasks hold >= 2 primitives each
+  uint32_t chunks;
+  uint32_t slots;    // tasks of more than one chunk
+  explicit SahSizes(uint32_t n)
+      : tasks(n / 2 + 2), chunks(tasks + n / kChunk + 2), slots(n / (kChunk + 1) + 2) {}
+  size_t bytes(uint32_t n) const {
+    return Scratch::padded((2 * size_t(n) - 1) * sizeof(DevBin)) +
+           Scratch::padded((2 * size_t(n) - 1) * 4) + 5 * Scratch::padded(size_t(n) * 4) +
+           2 * Scratch::padded(size_t(tasks) * sizeof(Task)) +
+           Scratch::padded(size_t(tasks) * sizeof(Split)) +
+           2 * Scratch::padded(size_t(tasks) * 8) + Scratch::padded(size_t(tasks) * 96) +
+           2 * Scratch::padded(size_t(chunks) * 4) + Scratch::padded(size_t(tasks) * 4) +
+           Scratch::padded(size_t(slots) * kBinWords * 4) + Scratch::padded(size_t(slots) * 4);
+  }
+};
+
 bool build_sah(Scratch& sc, const DevBin* prim, const uint32_t* d_bounds, uint32_t n,
                uint32_t max_leaf, cudaStream_t st, void* temp, size_t temp_bytes,
                uint64_t* h_total, BinTree& bt, std::string& err) {
   uint32_t total_nodes = 2 * n - 1;
-  uint32_t task_cap = n / 2 + 2;                   // open tasks hold >= 2 primitives each
-  uint32_t chunk_cap = task_cap + n / kChunk + 2;
-  uint32_t slot_cap = n / (kChunk + 1) + 2;        // tasks of more than one chunk
+  const SahSizes sizes(n);
+  const uint32_t task_cap = sizes.tasks, chunk_cap = sizes.chunks, slot_cap = sizes.slots;
   DevBin* nodes = sc.alloc<DevBin>(total_nodes, err);
   uint32_t* count = sc.alloc<uint32_t>(total_nodes, err);
   uint32_t* idx = sc.alloc<uint32_t>(n, err);
@@ -1040,7 +1094,8 @@ bool build_sah(Scratch& sc, const DevBin* prim, const uint32_t* d_bounds, uint32
 
 bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint32_t* h_tris,
                            uint32_t n, const BuildOptions& opts, DeviceBuilder method,
-                           cudaStream_t st, DeviceBvh& out, std::string& err, BinaryDump* dump) {
+                           cudaStream_t st, DeviceBvh& out, std::string& err, BinaryDump* dump,
+                           const ShadeInput* shading) {
   auto t0 = std::chrono::steady_clock::now();
   out = DeviceBvh();
   if(opts.max_leaf_tris < 1 || opts.max_leaf_tris > 2) {
@@ -1056,7 +1111,30 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
     err = "too many triangles for the device BVH build";
     return false;
   }
+  // temporary storage for CUB, sized for the largest call
+  size_t sort_bytes = 0, scan64 = 0, scan32 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint64_t*>(nullptr),
+                                  static_cast<uint64_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+                                  static_cast<uint32_t*>(nullptr), int(n), 0, 63, st);
+  cub::DeviceScan::InclusiveSum(nullptr, scan64, static_cast<uint64_t*>(nullptr),
+                                static_cast<uint64_t*>(nullptr), int(std::max(n, 2u)), st);
+  cub::DeviceScan::ExclusiveSum(nullptr, scan32, static_cast<uint32_t*>(nullptr),
+                                static_cast<uint32_t*>(nullptr), int(n), st);
+  size_t temp_bytes = std::max(sort_bytes, std::max(scan64, scan32));
+  const uint32_t level_cap = n / (opts.max_leaf_tris + 1) + 2;   // wide nodes of a level
   Scratch sc;
+  const size_t tri_words = Scratch::padded(4 * size_t(n));
+  if(!sc.reserve(Scratch::padded(12 * size_t(vert_count)) + Scratch::padded(12 * size_t(n)) +
+                 Scratch::padded(n * sizeof(DevBin)) + Scratch::padded(48) +
+                 Scratch::padded(temp_bytes) +
+                 (shading ? (shading->material ? tri_words : 0) +
+                            (shading->light ? tri_words : 0) : 0) +
+                 (method == DeviceBuilder::kPloc ? ploc_bytes(n) : SahSizes(n).bytes(n)) +
+                 4 * Scratch::padded(4 * size_t(level_cap)) +
+                 Scratch::padded(level_cap * sizeof(Plan)) +
+                 2 * Scratch::padded(8 * size_t(level_cap)) + Scratch::padded(4), err)) {
+    return false;
+  }
   float* verts = sc.alloc<float>(3 * size_t(vert_count), err);
   uint32_t* tris = sc.alloc<uint32_t>(3 * size_t(n), err);
   DevBin* prim = sc.alloc<DevBin>(n, err);
@@ -1079,16 +1157,25 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
   }
   k_prim_bounds<<<blocks_for(n, 256), 256, 0, st>>>(verts, tris, n, prim, bounds);
 
-  // temporary storage for CUB, sized for the largest call
-  size_t sort_bytes = 0, scan64 = 0, scan32 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint64_t*>(nullptr),
-                                  static_cast<uint64_t*>(nullptr), static_cast<uint32_t*>(nullptr),
-                                  static_cast<uint32_t*>(nullptr), int(n), 0, 63, st);
-  cub::DeviceScan::InclusiveSum(nullptr, scan64, static_cast<uint64_t*>(nullptr),
-                                static_cast<uint64_t*>(nullptr), int(std::max(n, 2u)), st);
-  cub::DeviceScan::ExclusiveSum(nullptr, scan32, static_cast<uint32_t*>(nullptr),
-                                static_cast<uint32_t*>(nullptr), int(n), st);
-  size_t temp_bytes = std::max(sort_bytes, std::max(scan64, scan32));
+  if(shading) {
+    const uint32_t* from[2] = {shading->material, shading->light};
+    uint32_t* words[2] = {nullptr, nullptr};
+    for(int k = 0; k < 2; ++k) {
+      if(!from[k]) { continue; }
+      words[k] = sc.alloc<uint32_t>(n, err);
+      if(!words[k] || !cuda_ok(cudaMemcpyAsync(words[k], from[k], 4 * size_t(n),
+                                               cudaMemcpyHostToDevice, st),
+                               "triangle material upload", err)) {
+        return false;
+      }
+    }
+    if(dev_alloc(&out.shade, 3 * size_t(n) * sizeof(float4)) != cudaSuccess) {
+      cudaGetLastError();
+      err = "cudaMalloc of the shading records failed";
+      return false;
+    }
+    k_shade<<<blocks_for(n, 256), 256, 0, st>>>(verts, tris, words[0], words[1], n, out.shade);
+  }
   void* temp = sc.alloc<unsigned char>(temp_bytes, err);
   PinnedWords pin;
   if(!temp ||
@@ -1136,7 +1223,6 @@ bool build_wide_bvh_device(const float* h_verts, uint32_t vert_count, const uint
   const DevBin* nodes = bt.nodes;
   const uint32_t* count = bt.count;
   uint32_t width = std::min(8u, std::max(2u, opts.width));
-  uint32_t level_cap = n / (opts.max_leaf_tris + 1) + 2;
   uint32_t* qbin = sc.alloc<uint32_t>(level_cap, err);
   uint32_t* qwide = sc.alloc<uint32_t>(level_cap, err);
   uint32_t* qbin2 = sc.alloc<uint32_t>(level_cap, err);

@@ -13,8 +13,8 @@
 //      pass opens candidates and assigns octant slots (bvh_wide.h, the same
 //      functions the host builder uses), a prefix sum of the internal-child
 //      and leaf-triangle counts gives every node its child_base / tri_base in
-//      breadth-first order, and an emit pass writes the quantized node (or
-//      its float-plane form) and the leaf triangles
+//      breadth-first order, and an emit pass writes the node as it is traversed and
+//      the leaf triangles
 //
 // The result depends only on the input (no atomics decide an order), and
 // collapsing the same binary tree on the host gives the same bytes.
@@ -31,23 +31,32 @@ namespace dort_gpu {
 enum class DeviceBuilder { kSah, kPloc };
 
 struct DeviceBvh {
-  void* nodes = nullptr;          // traversal nodes (WideNodeF, or WideNode when quantized)
+  void* nodes = nullptr;          // TraceNodes
   size_t node_bytes = 0;          // allocated bytes of `nodes`
   uint32_t node_count = 0;
   LeafTri* tris = nullptr;        // tri_count leaf triangles
+  float4* shade = nullptr;        // shading records (3 per triangle), when asked for
   uint32_t tri_count = 0;
   uint32_t depth = 0;             // levels of wide nodes
   uint32_t iterations = 0;        // SAH levels, or PLOC iterations
   double ms = 0.0;                // wall time of the build (uploads included)
 };
 
-// Builds the wide BVH of a host triangle mesh on the current device.  The
-// mesh must be valid (indices in range, finite coordinates of magnitude at
-// most 1e15: validate_mesh).  On success the caller owns out.nodes and
-// out.tris (cudaFree).
+// What the shading records hold beside the vertices: host arrays of a word per
+// triangle, null for all zero.
+struct ShadeInput {
+  const uint32_t* material;   // material index
+  const uint32_t* light;      // light index + 1, 0 if not emissive
+};
+
+// Builds the wide BVH of a host triangle mesh on the current device, and with
+// `shading` its shading records.  The mesh must be valid (indices in range,
+// finite coordinates of magnitude at most 1e15: validate_mesh).  The caller
+// owns out.nodes, out.tris and out.shade (cudaFree; on failure out.shade may
+// be set, the others are null).
 bool build_wide_bvh_device(const float* verts, uint32_t vert_count, const uint32_t* tris,
                            uint32_t tri_count, const BuildOptions& opts, DeviceBuilder method,
                            cudaStream_t stream, DeviceBvh& out, std::string& err,
-                           BinaryDump* dump = nullptr);
+                           BinaryDump* dump = nullptr, const ShadeInput* shading = nullptr);
 
 }  // namespace dort_gpu

@@ -127,16 +127,25 @@ static int upload(dort_scene* s, const std::vector<T>& v, const T** out) {
   return DORT_OK;
 }
 
-// Builds the BVH on the device (the scene owns the result).
-static int device_bvh(dort_scene* s, const dort_scene_desc* desc) {
+// Builds the BVH and the shading records on the device (the scene owns them).
+static int device_bvh(dort_scene* s, const dort_scene_desc* desc, const HostScene& hs) {
   BuildOptions opts;
   opts.width = desc->bvh_width ? desc->bvh_width : 8;
   DeviceBvh db;
   std::string err;
   DeviceBuilder method =
       desc->bvh_build == DORT_BVH_BUILD_PLOC ? DeviceBuilder::kPloc : DeviceBuilder::kSah;
-  if(!build_wide_bvh_device(desc->verts, desc->vert_count, desc->tris, desc->tri_count, opts,
-                            method, nullptr, db, err)) {
+  const ShadeInput shading{desc->tri_material,
+                           hs.tri_light.empty() ? nullptr : hs.tri_light.data()};
+  const bool ok = build_wide_bvh_device(desc->verts, desc->vert_count, desc->tris,
+                                        desc->tri_count, opts, method, nullptr, db, err, nullptr,
+                                        &shading);
+  if(db.shade) {
+    s->allocations.push_back(db.shade);
+    s->device_bytes += 3 * size_t(desc->tri_count) * sizeof(float4);
+    s->pt.shade = db.shade;
+  }
+  if(!ok) {
     int code = DORT_ERR_CUDA;
     if(err.rfind("cudaMalloc", 0) == 0 || err.find("out of memory") != std::string::npos) {
       code = DORT_ERR_OOM;
@@ -183,8 +192,9 @@ __global__ void leaf_tris_to_vertices(float4* tris, uint32_t count, const float4
 
 static int scene_upload(dort_scene* s, const dort_scene_desc* desc, const HostScene& hs) {
   int rc;
+  std::memset(&s->pt, 0, sizeof(s->pt));
   if(hs.device_bvh) {
-    if((rc = device_bvh(s, desc)) != DORT_OK) { return rc; }
+    if((rc = device_bvh(s, desc, hs)) != DORT_OK) { return rc; }
   } else {
     const unsigned char* nodes;
     const LeafTri* tris;
@@ -202,8 +212,7 @@ static int scene_upload(dort_scene* s, const dort_scene_desc* desc, const HostSc
   }
 
   PtScene& pt = s->pt;
-  std::memset(&pt, 0, sizeof(pt));
-  if((rc = upload(s, hs.shade, &pt.shade)) != DORT_OK) { return rc; }
+  if(!hs.device_bvh && (rc = upload(s, hs.shade, &pt.shade)) != DORT_OK) { return rc; }
   if(desc->flags & DORT_SCENE_WATERTIGHT) {
     if(s->trace.tri_count) {
       leaf_tris_to_vertices<<<std::min<uint32_t>((s->trace.tri_count + 255) / 256, 4096), 256>>>(

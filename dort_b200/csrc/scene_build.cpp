@@ -252,6 +252,8 @@ bool build_host_scene(const dort_scene_desc* desc, HostScene& hs, std::string& e
     return false;
   }
   hs.device_bvh = allow_device_bvh && desc->bvh_build != DORT_BVH_BUILD_HOST;
+  // bounds of the triangles
+  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   BuildOptions opts;
   opts.width = desc->bvh_width ? desc->bvh_width : 8;
   if(hs.device_bvh) {
@@ -259,7 +261,7 @@ bool build_host_scene(const dort_scene_desc* desc, HostScene& hs, std::string& e
       err = "bvh_width must be 2..8";
       return false;
     }
-    if(!validate_mesh(desc->verts, desc->vert_count, desc->tris, n, err)) { return false; }
+    if(!scan_mesh(desc->verts, desc->vert_count, desc->tris, n, lo, hi, err)) { return false; }
   } else {
     auto b0 = std::chrono::steady_clock::now();
     if(!build_wide_bvh(desc->verts, desc->vert_count, desc->tris, n, opts, hs.bvh, err)) {
@@ -270,16 +272,19 @@ bool build_host_scene(const dort_scene_desc* desc, HostScene& hs, std::string& e
   }
 
   // per-triangle shading records and area lights
-  hs.shade.assign(3 * size_t(n), make_float4(0.f, 0.f, 0.f, 0.f));
+  hs.shade.clear();
+  if(!hs.device_bvh) { hs.shade.resize(3 * size_t(n)); }
+  hs.tri_light.clear();
   hs.lights.clear();
   std::vector<float> powers;
   hs.emissive_count = 0;
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for(uint32_t t = 0; t < n; ++t) {
+  // with the records made on the device, plain triangles need no look here
+  const bool plain = hs.device_bvh && !desc->tri_material && !desc->tri_emission;
+  for(uint32_t t = 0; t < n && !plain; ++t) {
     const float* p[3];
     for(int k = 0; k < 3; ++k) {
       p[k] = desc->verts + 3 * size_t(desc->tris[3 * size_t(t) + k]);
-      for(int a = 0; a < 3; ++a) {
+      for(int a = 0; a < 3 && !hs.device_bvh; ++a) {
         lo[a] = std::min(lo[a], p[k][a]);
         hi[a] = std::max(hi[a], p[k][a]);
       }
@@ -323,8 +328,11 @@ bool build_host_scene(const dort_scene_desc* desc, HostScene& hs, std::string& e
         hs.lights.push_back(l);
         light = uint32_t(hs.lights.size());
         hs.emissive_count += 1;
+        if(hs.tri_light.empty()) { hs.tri_light.resize(n, 0u); }
+        hs.tri_light[t] = light;
       }
     }
+    if(hs.device_bvh) { continue; }
     uint32_t matbits, lightbits;
     std::memcpy(&matbits, &mat, 4);
     std::memcpy(&lightbits, &light, 4);

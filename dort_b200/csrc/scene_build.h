@@ -14,7 +14,8 @@ struct HostScene {
   WideBvh bvh;                       // empty when device_bvh (built on the device)
   bool device_bvh = false;
   double bvh_ms = 0.0;               // host BVH build time
-  std::vector<float4> shade;         // 3 per triangle
+  std::vector<float4> shade;         // 3 per triangle; empty when device_bvh (made there too)
+  std::vector<uint32_t> tri_light;   // light index + 1 per triangle; empty when none emits
   std::vector<DevMaterial> mats;
   std::vector<DevLight> lights;
   std::vector<float> light_cdf;

@@ -13,7 +13,7 @@ torch = pytest.importorskip("torch")
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kind", ["diff", "delt"])
+@pytest.mark.parametrize("kind", ["diff", "glos"])
 @pytest.mark.parametrize("per", [1, 3, 4, 5])
 def test_samples_per_thread(kind, per):
     w, h = 250, 130
