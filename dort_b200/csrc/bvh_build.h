@@ -4,12 +4,10 @@
 // (src/dort/bvh.cpp:9-416) and traverses it with a 64-entry stack of 32-byte
 // nodes (bvh.cpp:418-469).  The device scene instead uses a wide BVH (up to 8
 // children per node) with 8-bit quantized child boxes and octant-ordered
-// child slots, laid out for 128-bit loads:
+// child slots:
 //
-//   WideNode (80 bytes = 5 x uint4, 16-byte aligned, always 3 x 32-byte
-//   sectors):
-//     float    p[3]        origin of the quantization grid
-//     uint8_t  e[3]        biased power-of-two exponents of the grid step
+//   WideNode: the builders' form of a node
+//     float    p[3], s[3]  origin and steps of the quantization grid
 //     uint8_t  imask       bit s set: slot s is an internal child
 //     uint32_t child_base  node index of the first internal child; internal
 //                          children are contiguous, ordered by slot
@@ -18,11 +16,14 @@
 //                          node's triangles are its leaf slots' first ones in
 //                          slot order, then their second ones
 //     uint8_t  qlo[3][8], qhi[3][8]   quantized child boxes
+//   TraceNode: the same as the device traverses it (three 32-byte loads)
 //
-// Child boxes are quantized outward with one full grid step of margin on
-// every side, so that the device slab test (rounded float arithmetic) never
-// culls a child that contains a hit.  The device traverses TraceNode (below):
-// the same nodes, laid out for three 32-byte loads.
+// Child boxes are quantized outward with a margin that covers the rounding of
+// the device slab test and of the triangle test (bvh_wide.h), so that no
+// child that contains a hit is culled.  (One grid step of margin on a
+// power-of-two grid, the form before, made the boxes larger: 4M camera rays on
+// the 1M-triangle soup 1.59 against 1.51 ms, 3M shadow rays on a 250k-triangle
+// sphere 0.90 against 0.85 ms.)
 //
 //   Triangle (48 bytes = 3 x float4, leaf order):
 //     (p0.xyz, original triangle index as bits), (e1.xyz, 0), (e2.xyz, 0)
@@ -40,9 +41,9 @@ namespace dort_gpu {
 void alloc_checkpoint();
 
 
-struct alignas(16) WideNode {
+struct WideNode {
   float p[3];
-  uint8_t e[3];
+  float s[3];
   uint8_t imask;
   uint32_t child_base;
   uint32_t tri_base;
@@ -50,12 +51,11 @@ struct alignas(16) WideNode {
   uint8_t qlo[3][8];
   uint8_t qhi[3][8];
 };
-static_assert(sizeof(WideNode) == 80, "WideNode must be 80 bytes");
 
 // The same node as the device traverses it.  96 bytes = three 32-byte loads.
 struct alignas(32) TraceNode {
   float p[3];            // origin of the quantization grid
-  float s[3];            // its steps (powers of two)
+  float s[3];            // its steps
   uint32_t child_base;
   uint32_t tri_base;
   uint32_t masks;        // bits 0..7: imask; bit 16 + 8 k + s: slot s is a leaf of more than k triangles

@@ -10,7 +10,7 @@
 //                     is scored by how far the candidate's centre lies in the
 //                     slot's octant direction from the node's centre; the
 //                     lowest score is taken first
-//   quantize_axis     8-bit conservative child planes on a power-of-two grid
+//   quantize_axis     8-bit conservative child planes on a grid of the node
 //   pack_trace_node   the quantized node in the layout the device traverses
 //
 // Every double product and sum is rounded on its own (BW_MUL / BW_ADD /
@@ -120,43 +120,40 @@ BW_HD void assign_slots(const A& acc, const uint32_t* cands, uint32_t n, float n
   }
 }
 
-// Picks the quantization grid of one axis: step 2^e, origin p one step below
-// the node's lower bound, 253 steps covering the extent; every child plane
-// encloses its child with at least one step of margin.  Returns false if the
-// exponent cannot be represented.
-BW_HD bool quantize_axis(float node_lo, float node_hi, const float* clo, const float* chi,
-                         int n, float& p_out, uint8_t& e_out, uint8_t* qlo, uint8_t* qhi) {
-  double lo = node_lo, hi = node_hi;
-  double ext = BW_SUB(hi, lo);
-  double mag = fmax(fabs(lo), fabs(hi));
-  double min_step = fmax(BW_MUL(mag, ldexp(1.0, -20)), ldexp(1.0, -100));
-  double step = fmax(ext / 253.0, min_step);
-  int ex;
-  double m = frexp(step, &ex);       // step = m 2^ex, m in [0.5, 1)
-  int e = m == 0.5 ? ex - 1 : ex;    // ceil(log2(step))
-  for(int attempt = 0; attempt < 8; ++attempt, ++e) {
-    if(e + 127 < 1 || e + 127 > 254) { return false; }
-    double s = ldexp(1.0, e);
-    double pd = BW_SUB(lo, s);
+// Picks the quantization grid of one axis: origin p, step s, and for every
+// child planes that enclose it with `margin` to spare (and 1/32 of a step, for
+// the rounding of the device's decoding).  253 steps cover the extent.
+// Returns false if no step fits.
+BW_HD bool quantize_axis(float node_lo, float node_hi, double margin, const float* clo,
+                         const float* chi, int n, float& p_out, float& s_out, uint8_t* qlo,
+                         uint8_t* qhi) {
+  const double lo = BW_SUB(double(node_lo), margin), hi = BW_ADD(double(node_hi), margin);
+  const double mag = fmax(fabs(lo), fabs(hi));
+  const double min_step = fmax(BW_MUL(mag, ldexp(1.0, -20)), ldexp(1.0, -100));
+  double step = fmax(BW_SUB(hi, lo) / 253.0, min_step);
+  for(int attempt = 0; attempt < 8; ++attempt, step = BW_MUL(step, 1.03125)) {
+    float sf = float(step);
+    if(double(sf) < step) { sf = nextafterf(sf, INFINITY); }
+    const double s = double(sf);
+    if(!(s <= 1e30)) { return false; }
+    const double spare = BW_ADD(margin, BW_MUL(s, 0.03125));
+    const double pd = BW_SUB(double(node_lo), spare);
     float pf = float(pd);
     if(double(pf) > pd) { pf = nextafterf(pf, -INFINITY); }
+    const double p = double(pf);
     bool ok = true;
     for(int i = 0; i < n && ok; ++i) {
-      double ql = BW_SUB(floor(BW_SUB(double(clo[i]), double(pf)) / s), 1.0);
-      double qh = BW_ADD(ceil(BW_SUB(double(chi[i]), double(pf)) / s), 1.0);
+      const double wlo = BW_SUB(double(clo[i]), spare), whi = BW_ADD(double(chi[i]), spare);
+      double ql = floor(BW_SUB(wlo, p) / s), qh = ceil(BW_SUB(whi, p) / s);
+      if(BW_ADD(p, BW_MUL(ql, s)) > wlo) { ql = BW_SUB(ql, 1.0); }
+      if(BW_ADD(p, BW_MUL(qh, s)) < whi) { qh = BW_ADD(qh, 1.0); }
       if(ql < 0.0 || qh > 255.0) { ok = false; break; }
-      double margin = BW_MUL(s, 0.999);
-      if(BW_ADD(double(pf), BW_MUL(ql, s)) > BW_SUB(double(clo[i]), margin) ||
-         BW_ADD(double(pf), BW_MUL(qh, s)) < BW_ADD(double(chi[i]), margin)) {
-        ok = false;
-        break;
-      }
       qlo[i] = uint8_t(ql);
       qhi[i] = uint8_t(qh);
     }
     if(ok) {
       p_out = pf;
-      e_out = uint8_t(e + 127);
+      s_out = sf;
       return true;
     }
   }
@@ -176,9 +173,15 @@ BW_HD bool quantize_node(const A& acc, const uint32_t* cands, const int cand_in_
       chi[a][s] = c >= 0 ? acc.hi(cands[c])[a] : nlo[a];
     }
   }
+  // The boxes' margin: 2^-14 of the node's largest coordinate, for the rounding
+  // of the triangle test (a few 2^-24 of the distance to the triangle), which
+  // may report hits that miss the exact box by that.
+  double mag = 0.0;
+  for(int a = 0; a < 3; ++a) { mag = fmax(mag, fmax(fabs(double(nlo[a])), fabs(double(nhi[a])))); }
+  const double margin = BW_MUL(mag, ldexp(1.0, -14));
   for(int a = 0; a < 3; ++a) {
-    if(!quantize_axis(nlo[a], nhi[a], clo[a], chi[a], 8, node.p[a], node.e[a], node.qlo[a],
-                      node.qhi[a])) {
+    if(!quantize_axis(nlo[a], nhi[a], margin, clo[a], chi[a], 8, node.p[a], node.s[a],
+                      node.qlo[a], node.qhi[a])) {
       return false;
     }
   }
@@ -194,7 +197,7 @@ BW_HD bool quantize_node(const A& acc, const uint32_t* cands, const int cand_in_
 BW_HD void pack_trace_node(const WideNode& n, TraceNode& t) {
   for(int a = 0; a < 3; ++a) {
     t.p[a] = n.p[a];
-    t.s[a] = float(ldexp(1.0, int(n.e[a]) - 127));
+    t.s[a] = n.s[a];
     for(int h = 0; h < 2; ++h) {
       uint32_t lo = 0, hi = 0;
       for(int j = 0; j < 4; ++j) {
