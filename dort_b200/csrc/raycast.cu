@@ -24,6 +24,7 @@ struct RaycastQueue {
   uint32_t* __restrict__ out_prim;
   float* __restrict__ out_tb;
   __device__ __forceinline__ const TraceScene& scene() const { return sc; }
+  __device__ __forceinline__ void take(int) const {}
   __device__ __forceinline__ void load(uint32_t i, TravState& s) const {
     float4 r0 = __ldcs(rays + 2 * size_t(i));
     float4 r1 = __ldcs(rays + 2 * size_t(i) + 1);

@@ -315,6 +315,30 @@ DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint3
   return ~miss & 0xffu;
 }
 
+// The same test for slot `slot` alone (a lane per slot, trace_wide).
+DG_HD bool slot_hit(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
+                    uint32_t slot, float ox, float oy, float oz, float ix, float iy, float iz,
+                    float t_min, float t_far_max) {
+  const float ax = DG_AS_FLOAT(n0[3]) * ix, ay = DG_AS_FLOAT(n0[4]) * iy,
+              az = DG_AS_FLOAT(n0[5]) * iz;
+  const float bx = DG_FMA(-32768.f, ax, (DG_AS_FLOAT(n0[0]) - ox) * ix);
+  const float by = DG_FMA(-32768.f, ay, (DG_AS_FLOAT(n0[1]) - oy) * iy);
+  const float bz = DG_FMA(-32768.f, az, (DG_AS_FLOAT(n0[2]) - oz) * iz);
+  const bool h = slot >= 4u, nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
+  const uint32_t lo_x = h ? n1[3] : n1[2], hi_x = h ? n1[5] : n1[4];
+  const uint32_t lo_y = h ? n1[7] : n1[6], hi_y = h ? n2[1] : n2[0];
+  const uint32_t lo_z = h ? n2[3] : n2[2], hi_z = h ? n2[5] : n2[4];
+  const uint32_t one = n1[1], j = slot & 3u;
+  const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(nx ? hi_x : lo_x, one, j), ax, bx),
+                           DG_FMA(DG_BYTE_FLOAT(ny ? hi_y : lo_y, one, j), ay, by),
+                           DG_FMA(DG_BYTE_FLOAT(nz ? hi_z : lo_z, one, j), az, bz));
+  float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT(nx ? lo_x : hi_x, one, j), ax, bx),
+                     DG_FMA(DG_BYTE_FLOAT(ny ? lo_y : hi_y, one, j), ay, by),
+                     DG_FMA(DG_BYTE_FLOAT(nz ? lo_z : hi_z, one, j), az, bz));
+  tf = DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, tf);
+  return (DG_AS_UINT(DG_MIN3(tf - tn, tf - t_min, t_far_max - tn)) >> 31) == 0u;
+}
+
 // Traversal state of one ray.  trav_node visits one node, trav_tri tests one
 // triangle, trav_step does a node and its triangles; trace_ray runs the steps
 // of one ray to the end, trace_queue (trace_queue.cuh) those of a whole queue.
@@ -420,28 +444,24 @@ DG_HD bool leaf_empty(uint2 leaf) { return (leaf.y & 0xffffu) == 0u; }
 // stack as soon as it is empty).
 DG_HD bool group_left(const TravState& s) { return (s.group.y & 0xffu) != 0u; }
 
-// Visits the next node (there must be one, group_left): its hit children
-// become the current group, its hit leaf slots are returned.
-template<class Stack>
-DG_HD uint2 trav_node(TravState& s, const TraceScene& sc, Stack& stack) {
-  // the hit child nearest in octant order: prefer the near half by slot bit
-  // 2, then bit 1, then bit 0
+// Takes the next node off the current group (there must be one, group_left):
+// the hit child nearest in octant order, that is, the near half by slot bit 2,
+// then bit 1, then bit 0.
+DG_HD const uint4* trav_next(TravState& s, const TraceScene& sc) {
   uint32_t pick = s.group.y & 0xffu;
   pick = (pick & s.near4) ? pick & s.near4 : pick;
   pick = (pick & s.near2) ? pick & s.near2 : pick;
   pick = (pick & s.near1) ? pick & s.near1 : pick;
   s.group.y ^= pick;
-  uint32_t node_idx = s.group.x + DG_POPC((s.group.y >> 8) & (pick - 1u));
+  const uint32_t node = s.group.x + DG_POPC((s.group.y >> 8) & (pick - 1u));
+  return sc.nodes + kNodeWords * size_t(node);
+}
 
-  const uint4* np = sc.nodes + kNodeWords * size_t(node_idx);
-  uint32_t n0[8], n1[8], n2[8];
-  load_32(np, n0);
-  load_32(np + 2, n1);
-  load_32(np + 4, n2);
-  const uint32_t hits = node_hits(n0, n1, n2, s.ox, s.oy, s.oz, s.ix, s.iy, s.iz, s.t_min,
-                                  DG_FMA(fabsf(s.best.t), DORT_SLAB_FAR_WIDEN, s.best.t));
-  const uint32_t child_base = n0[6], tri_base = n0[7], masks = n1[0];
-
+// Goes on from a node with the slots `hits`: its internal ones become the
+// current group, its leaf ones are returned.
+template<class Stack>
+DG_HD uint2 trav_enter(TravState& s, Stack& stack, uint32_t hits, uint32_t child_base,
+                       uint32_t tri_base, uint32_t masks) {
   const uint32_t inner = hits & masks & 0xffu;
   if(inner) {
     if(group_left(s)) {
@@ -454,6 +474,20 @@ DG_HD uint2 trav_node(TravState& s, const TraceScene& sc, Stack& stack) {
     s.group = stack.pop(--s.sp);
   }
   return make_uint2(tri_base, (masks & 0xffff0000u) | ((hits * 0x101u) & (masks >> 16)));
+}
+
+// Visits the next node: its hit children become the current group, its hit
+// leaf slots are returned.
+template<class Stack>
+DG_HD uint2 trav_node(TravState& s, const TraceScene& sc, Stack& stack) {
+  const uint4* np = trav_next(s, sc);
+  uint32_t n0[8], n1[8], n2[8];
+  load_32(np, n0);
+  load_32(np + 2, n1);
+  load_32(np + 4, n2);
+  const uint32_t hits = node_hits(n0, n1, n2, s.ox, s.oy, s.oz, s.ix, s.iy, s.iz, s.t_min,
+                                  DG_FMA(fabsf(s.best.t), DORT_SLAB_FAR_WIDEN, s.best.t));
+  return trav_enter(s, stack, hits, n0[6], n0[7], n1[0]);
 }
 
 // Tests the next triangle of a non-empty `leaf`; true when it was hit (and

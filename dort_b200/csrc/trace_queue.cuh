@@ -95,6 +95,110 @@ struct WarpBuffer {
   }
 };
 
+// The last few rays of a warp (at most kWideRays, in the lanes `busy`), eight
+// lanes to a ray: every lane of a group holds its ray's whole state and walks
+// the tree in step with the others; lane j tests the box of slot j and the
+// triangles of leaf slot j, and votes and shuffles bring the results together.
+// A lone ray's steps are chains of dependent instructions; this way a node
+// costs some 90 of them instead of 270 and a node's triangles one test or two.
+// The results are those of one lane: the same boxes pass, and the closest hit
+// is the minimum whatever the order.
+constexpr int kWideRays = 4;
+
+template<bool ANY_HIT, bool EXACT_MT, int WT, class Q, class Stack>
+__device__ __forceinline__ void trace_wide(Q& q, TravState& s, Stack& stack, uint2 leaf,
+                                           uint2 leaf2, uint32_t item, uint32_t busy) {
+  const uint32_t lane = threadIdx.x & 31u, slot = lane & 7u, group = lane & 24u;
+  // group k takes the k-th busy lane's ray
+  uint32_t from = busy;
+  for(uint32_t k = 0; k < (lane >> 3); ++k) { from &= from - 1u; }
+  const int src = from ? __ffs(from) - 1 : int(lane);
+  auto take = [&](auto& v) { v = __shfl_sync(kWarpAll, v, src); };
+  take(s.ox); take(s.oy); take(s.oz);
+  take(s.dx); take(s.dy); take(s.dz);
+  take(s.t_min);
+  take(s.ix); take(s.iy); take(s.iz);
+  take(s.near4); take(s.near2); take(s.near1);
+  take(s.best.t); take(s.best.b1); take(s.best.b2); take(s.best.prim);
+  take(s.group.x); take(s.group.y);
+  if(WT != kTriMt) {
+    take(s.wt.kx); take(s.wt.ky); take(s.wt.kz);
+    take(s.wt.sx); take(s.wt.sy); take(s.wt.sz);
+  }
+  take(leaf.x); take(leaf.y); take(leaf2.x); take(leaf2.y);
+  take(item);
+  q.take(src);
+  if(!from) { item = kNoItem; }
+  const int had = s.sp;
+  take(s.sp);
+  const int deepest = __reduce_max_sync(kWarpAll, had);
+  for(int k = 0; k < deepest; ++k) {
+    uint2 e = k < had ? stack.pop(k) : make_uint2(0u, 0u);
+    take(e.x);
+    take(e.y);
+    if(k < s.sp) { stack.push(k, e); }
+  }
+  for(;;) {
+    const bool live = item != kNoItem;
+    // the pending triangles: first ones, then second ones
+    if(__any_sync(kWarpAll, live && !leaf_empty(leaf))) {
+      bool hit = false;
+#pragma unroll
+      for(uint32_t k = 0; k < 2; ++k) {
+        uint2 one = make_uint2(leaf.x, leaf.y & (0xffff0000u | (1u << (8u * k + slot))));
+        if(live && !leaf_empty(one)) {
+          if(trav_tri<ANY_HIT, EXACT_MT, WT>(s, q.scene(), one)) { hit = true; }
+        }
+      }
+      const uint32_t hits = __ballot_sync(kWarpAll, hit);
+      if(hits) {
+#pragma unroll
+        for(int d = 1; d < 8; d <<= 1) {
+          Hit o;
+          o.t = __shfl_xor_sync(kWarpAll, s.best.t, d);
+          o.b1 = __shfl_xor_sync(kWarpAll, s.best.b1, d);
+          o.b2 = __shfl_xor_sync(kWarpAll, s.best.b2, d);
+          o.prim = __shfl_xor_sync(kWarpAll, s.best.prim, d);
+          if(o.prim != kMiss && (s.best.prim == kMiss || o.t < s.best.t ||
+                                 (o.t == s.best.t && o.prim > s.best.prim))) {
+            s.best = o;
+          }
+        }
+      }
+      leaf = leaf2;
+      leaf2.y = 0u;
+      if(ANY_HIT && ((hits >> group) & 0xffu)) {
+        leaf.y = 0u;
+        s.group.y = 0u;
+        s.sp = 0;
+      }
+    }
+    const bool go = live && group_left(s) && leaf_empty(leaf);
+    bool box = false;
+    uint32_t child_base = 0, tri_base = 0, masks = 0;
+    if(go) {
+      const uint4* np = trav_next(s, q.scene());
+      uint32_t n0[8], n1[8], n2[8];
+      load_32(np, n0);
+      load_32(np + 2, n1);
+      load_32(np + 4, n2);
+      child_base = n0[6];
+      tri_base = n0[7];
+      masks = n1[0];
+      box = slot_hit(n0, n1, n2, slot, s.ox, s.oy, s.oz, s.ix, s.iy, s.iz, s.t_min,
+                     fmaf(fabsf(s.best.t), DORT_SLAB_FAR_WIDEN, s.best.t));
+    }
+    const uint32_t hits = (__ballot_sync(kWarpAll, box) >> group) & 0xffu;
+    if(go) { leaf = trav_enter(s, stack, hits, child_base, tri_base, masks); }
+    const bool mine = live && !group_left(s) && leaf_empty(leaf);
+    if(__any_sync(kWarpAll, mine)) {
+      q.done(mine && slot == 0u, item, s);
+      if(mine) { item = kNoItem; }
+      if(__all_sync(kWarpAll, item == kNoItem)) { return; }
+    }
+  }
+}
+
 // Traces the entries [0, count) of a queue.  Every warp starts with the chunk
 // of its own number; `cursor` (zero before) counts the entries taken after
 // those, and is left alone by queues that the first chunks cover.
@@ -103,6 +207,7 @@ struct WarpBuffer {
 //   void load(uint32_t i, TravState& s)     starts the ray of entry i
 //   void done(bool mine, uint32_t i, const TravState& s)
 //     called by the whole warp; lanes with `mine` have finished entry i (s.best)
+//   void take(int src)                      the lane's own state becomes lane src's
 template<bool ANY_HIT, bool EXACT_MT, int WT, class Q>
 __device__ __forceinline__ void trace_queue(Q& q, uint32_t count, uint32_t* cursor) {
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -139,6 +244,15 @@ __device__ __forceinline__ void trace_queue(Q& q, uint32_t count, uint32_t* curs
         next += __popc(idle);
       } else if(idle == kWarpAll) {
         break;
+      }
+      if(next >= end && !more) {
+        const uint32_t busy = __ballot_sync(kWarpAll, item != kNoItem);
+        if(__popc(busy) <= kWideRays) {
+          if(busy) {
+            trace_wide<ANY_HIT, EXACT_MT, WT>(q, s, stack, leaf, leaf2, item, busy);
+          }
+          break;
+        }
       }
     }
     // node steps; a lane with two nodes' triangles waits

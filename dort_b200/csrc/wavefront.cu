@@ -600,6 +600,7 @@ struct LaneScene {
   const PtScene* sc;
   __device__ __forceinline__ explicit LaneScene(const J& jobs) : sc(&jobs.scene(0)) {}
   __device__ __forceinline__ void select(const J&, const WfDev&, uint32_t) {}
+  __device__ __forceinline__ void take(int) {}
   __device__ __forceinline__ const PtScene& pt() const { return *sc; }
   __device__ __forceinline__ const TraceScene& trace() const { return sc->trace; }
 };
@@ -611,6 +612,11 @@ struct LaneScene<J, true> {
       : sc(&jobs.scene(0)), tr(sc->trace) {}
   __device__ __forceinline__ void select(const J& jobs, const WfDev& w, uint32_t slot) {
     sc = &jobs.scene(w.meta[slot].w >> 8);
+    tr = sc->trace;
+  }
+  __device__ __forceinline__ void take(int src) {
+    sc = reinterpret_cast<const PtScene*>(
+        __shfl_sync(kWarpAll, reinterpret_cast<unsigned long long>(sc), src));
     tr = sc->trace;
   }
   __device__ __forceinline__ const PtScene& pt() const { return *sc; }
@@ -645,6 +651,10 @@ struct ExtendQueue {
     scene_of.select(jobs, w, slot);
     const Pair r = load_pair(w.ray + slot);
     trav_init(s, scene(), r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, INFINITY);
+  }
+  __device__ __forceinline__ void take(int src) {
+    slot = __shfl_sync(kWarpAll, slot, src);
+    scene_of.take(src);
   }
   __device__ __forceinline__ void done(bool mine, uint32_t, const TravState& s) {
     uint32_t prim = kMiss;
@@ -1036,6 +1046,10 @@ struct ShadowQueue {
     t_max = d.w;
     trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, d.w);
   }
+  __device__ __forceinline__ void take(int src) {
+    t_max = __shfl_sync(kWarpAll, t_max, src);
+    scene_of.take(src);
+  }
   __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) {
     const bool open = mine &&
                       with_shapes<true, J::kGeneral>(scene_of.pt(), s, t_max).prim == kMiss;
@@ -1171,6 +1185,7 @@ struct NeebQueue {
     const float4 o = w.nb_o[i], d = w.nb_d[i];
     trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, INFINITY);
   }
+  __device__ __forceinline__ void take(int src) { scene_of.take(src); }
   __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) {
     if(!mine) { return; }
     const PtScene& sc = scene_of.pt();
