@@ -270,6 +270,21 @@ __device__ __forceinline__ void adj_record(WfDev& w, uint32_t slot, uint32_t kin
   }
 }
 
+// Appends `slot` to the shade queue of its `kind` (kShadeQueues: to none).  The
+// counters of all kinds are added to by one instruction, a lane for each kind
+// that occurs, so that the warp waits for one atomic and not for up to six.
+__device__ __forceinline__ void append_by_kind(WfDev& w, uint32_t kind, uint32_t slot) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t same = __match_any_sync(0xffffffffu, kind);
+  const uint32_t leader = __ffs(same) - 1u;
+  uint32_t base = 0;
+  if(kind < kShadeQueues && lane == leader) {
+    base = atomicAdd(ctr_at(w.ctr, C_KQ0 + kind), __popc(same));
+  }
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if(kind < kShadeQueues) { w.kq[kind][base + __popc(same & ((1u << lane) - 1u))] = slot; }
+}
+
 __device__ __forceinline__ uint32_t wave_of(const WfDev& w) {
   return *(volatile uint32_t*)ctr_at(w.ctr, C_WAVES);
 }
@@ -577,12 +592,7 @@ __global__ void wf_classify(WfDev w) {
       slot = act[i];
       kind = w.hit_kind[slot];
     }
-#pragma unroll
-    for(uint32_t k = 0; k < kShadeQueues; ++k) {
-      bool mine = kind == k;
-      uint32_t at = warp_append(ctr_at(w.ctr, C_KQ0 + k), mine);
-      if(mine) { w.kq[k][at] = slot; }
-    }
+    append_by_kind(w, kind, slot);
   }
 }
 
@@ -682,12 +692,7 @@ struct ExtendQueue {
       if(have) { w.hit_kind[sl] = kind; }
       return;
     }
-#pragma unroll
-    for(uint32_t k = 0; k < kShadeQueues; ++k) {
-      bool mine = kind == k;
-      uint32_t at = warp_append(ctr_at(w.ctr, C_KQ0 + k), mine);
-      if(mine) { w.kq[k][at] = sl; }
-    }
+    append_by_kind(w, kind, sl);
   }
 };
 
@@ -857,6 +862,7 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
     n += qn[k];
   }
   const uint32_t req_nd = F_ALL & ~F_DELTA;
+  const uint32_t lane = threadIdx.x & 31u;
   for(;;) {
     uint32_t base = warp_fetch(ctr_at(w.ctr, C_F_SHADE));
     if(base >= n) { break; }
@@ -986,22 +992,36 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
     }
     (void)cont;
     (void)done;
-    uint32_t si = warp_append(ctr_at(w.ctr, C_SHADOW), nee.sh);
+    // the entries of the shadow queue (both strategies) and of the BSDF-strategy
+    // queue: one atomic a queue, both at once
+    const uint32_t m1 = __ballot_sync(0xffffffffu, nee.sh);
+    const uint32_t m2 = __ballot_sync(0xffffffffu, nee.sh2);
+    const uint32_t m3 = __ballot_sync(0xffffffffu, nee.nb);
+    const uint32_t n1 = __popc(m1);
+    uint32_t at = 0;
+    if(lane < 2u) {
+      const uint32_t add = lane == 0u ? n1 + __popc(m2) : uint32_t(__popc(m3));
+      if(add) { at = atomicAdd(ctr_at(w.ctr, C_SHADOW + lane), add); }
+    }
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t sh_base = __shfl_sync(0xffffffffu, at, 0);
+    const uint32_t nb_base = __shfl_sync(0xffffffffu, at, 1);
     if(nee.sh) {
+      const uint32_t si = sh_base + __popc(m1 & lt);
       w.sh_slot[si] = slot;
       w.sh_o[si] = nee.sh_o;
       w.sh_d[si] = nee.sh_d;
       w.sh_c[si] = nee.sh_c;
     }
-    uint32_t si2 = warp_append(ctr_at(w.ctr, C_SHADOW), nee.sh2);
     if(nee.sh2) {
-      w.sh_slot[si2] = slot;
-      w.sh_o[si2] = nee.sh2_o;
-      w.sh_d[si2] = nee.sh2_d;
-      w.sh_c[si2] = nee.sh2_c;
+      const uint32_t si = sh_base + n1 + __popc(m2 & lt);
+      w.sh_slot[si] = slot;
+      w.sh_o[si] = nee.sh2_o;
+      w.sh_d[si] = nee.sh2_d;
+      w.sh_c[si] = nee.sh2_c;
     }
-    uint32_t ni = warp_append(ctr_at(w.ctr, C_NEEB), nee.nb);
     if(nee.nb) {
+      const uint32_t ni = nb_base + __popc(m3 & lt);
       w.nb_slot[ni] = slot;
       w.nb_o[ni] = nee.nb_o;
       w.nb_d[ni] = nee.nb_d;
