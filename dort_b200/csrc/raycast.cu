@@ -25,6 +25,9 @@ struct RaycastQueue {
   float* __restrict__ out_tb;
   __device__ __forceinline__ const TraceScene& scene() const { return sc; }
   __device__ __forceinline__ void take(int) const {}
+  __device__ __forceinline__ void ahead(uint32_t first, uint32_t end) const {
+    prefetch_l2(rays + 2 * size_t(first), rays + 2 * size_t(end), threadIdx.x & 31u);
+  }
   __device__ __forceinline__ void load(uint32_t i, TravState& s) const {
     float4 r0 = __ldcs(rays + 2 * size_t(i));
     float4 r1 = __ldcs(rays + 2 * size_t(i) + 1);

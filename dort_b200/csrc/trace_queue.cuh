@@ -27,6 +27,13 @@ namespace dort_gpu {
 constexpr uint32_t kNoItem = 0xffffffffu;
 constexpr uint32_t kWarpAll = 0xffffffffu;
 
+// Brings the bytes of [from, to) on their way to the L2 cache, a 128-byte line
+// per lane of `lanes` (the first ones).
+__device__ __forceinline__ void prefetch_l2(const void* from, const void* to, uint32_t lane) {
+  const char* p = static_cast<const char*>(from) + 128u * lane;
+  if(p < to) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
+}
+
 constexpr int kTriLanes = 16;
 constexpr int kMinLanes = 8;
 constexpr int kIdleLanes = 4;
@@ -208,6 +215,7 @@ __device__ __forceinline__ void trace_wide(Q& q, TravState& s, Stack& stack, uin
 //   void done(bool mine, uint32_t i, const TravState& s)
 //     called by the whole warp; lanes with `mine` have finished entry i (s.best)
 //   void take(int src)                      the lane's own state becomes lane src's
+//   void ahead(uint32_t first, uint32_t end)   entries the warp will start soon
 template<bool ANY_HIT, bool EXACT_MT, int WT, class Q>
 __device__ __forceinline__ void trace_queue(Q& q, uint32_t count, uint32_t* cursor) {
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
@@ -234,6 +242,7 @@ __device__ __forceinline__ void trace_queue(Q& q, uint32_t count, uint32_t* curs
         next = warps * first + __shfl_sync(kWarpAll, b, 0);
         end = min(next + want, count);
         more = next < count;
+        q.ahead(next, end);
       }
       if(next < end) {
         const uint32_t at = next + __popc(idle & lt);

@@ -662,6 +662,7 @@ struct ExtendQueue {
     const Pair r = load_pair(w.ray + slot);
     trav_init(s, scene(), r.a.x, r.a.y, r.a.z, r.a.w, r.b.x, r.b.y, r.b.z, INFINITY);
   }
+  __device__ __forceinline__ void ahead(uint32_t, uint32_t) const {}
   __device__ __forceinline__ void take(int src) {
     slot = __shfl_sync(kWarpAll, slot, src);
     scene_of.take(src);
@@ -1066,6 +1067,11 @@ struct ShadowQueue {
     t_max = d.w;
     trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, d.w);
   }
+  __device__ __forceinline__ void ahead(uint32_t first, uint32_t end) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    prefetch_l2(w.sh_o + first, w.sh_o + end, lane);
+    prefetch_l2(w.sh_d + first, w.sh_d + end, lane);
+  }
   __device__ __forceinline__ void take(int src) {
     t_max = __shfl_sync(kWarpAll, t_max, src);
     scene_of.take(src);
@@ -1204,6 +1210,11 @@ struct NeebQueue {
     if(J::kBatched) { scene_of.select(jobs, w, w.nb_slot[i]); }
     const float4 o = w.nb_o[i], d = w.nb_d[i];
     trav_init(s, scene(), o.x, o.y, o.z, o.w, d.x, d.y, d.z, INFINITY);
+  }
+  __device__ __forceinline__ void ahead(uint32_t first, uint32_t end) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    prefetch_l2(w.nb_o + first, w.nb_o + end, lane);
+    prefetch_l2(w.nb_d + first, w.nb_d + end, lane);
   }
   __device__ __forceinline__ void take(int src) { scene_of.take(src); }
   __device__ __forceinline__ void done(bool mine, uint32_t i, const TravState& s) {
