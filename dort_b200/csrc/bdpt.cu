@@ -45,12 +45,13 @@ constexpr uint32_t kBdptChunk = 1u << DORT_BDPT_CHUNK_LOG2;
 // Resident blocks per SM the register allocation must allow (Cornell
 // workload, A/B against the compiler's 104-128 registers): connection
 // kernels at 6 blocks +13 %, at 8 (64 registers, some spill) another +4 %;
-// walk kernels at 5 (96 registers) +8 %, at 6 less.
+// walk kernels at 5 (96 registers) +8 %, and at 6 (80) once the traversal took
+// fewer registers (see bd_trace in bdpt.cuh).
 #ifndef DORT_BDPT_CONNECT_MIN_BLOCKS
 #define DORT_BDPT_CONNECT_MIN_BLOCKS 8
 #endif
 #ifndef DORT_BDPT_WALK_MIN_BLOCKS
-#define DORT_BDPT_WALK_MIN_BLOCKS 5
+#define DORT_BDPT_WALK_MIN_BLOCKS 6
 #endif
 
 // Connection slots of one sample: (s, t) with t >= 1 and s + t <= D =

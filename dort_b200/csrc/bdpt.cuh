@@ -24,19 +24,23 @@ constexpr uint32_t kBdptVerts = 16;   // vertices per walk: max_depth <= 13
 // they were called out of line.  Each device kernel now runs one walk kind or
 // one connection case, small enough to inline them: 148.8 against 136.5 M
 // samples/s on the Cornell workload.  DORT_BD_NOINLINE keeps them out of
-// line.
+// line.  Only the connections' ray queries are calls (path_trace): the kernels
+// are still bound by instruction fetch and 64 registers, and so the rest of a
+// connection keeps its registers around the traversal (256x256 Cornell box with
+// Phong surfaces at 16 spp, depth 8, together with 6 instead of 5 walk blocks per
+// SM: 5.92 -> 5.55 ms; with the walks' own queries as calls 6.02).
 #ifdef DORT_BD_NOINLINE
 #define DORT_BD_FN __host__ __device__ __noinline__
 #else
 #define DORT_BD_FN DG_HD
 #endif
-template<bool ANY_HIT, bool G>
+template<bool ANY_HIT, bool G, int kCalls>
 DORT_BD_FN Hit bd_trace(const PtScene& sc, V3 o, float t_min, V3 d, float t_max) {
-  return scene_trace<ANY_HIT, G>(sc, o, t_min, d, t_max);
+  return path_trace<ANY_HIT, G, kCalls>(sc, o, t_min, d, t_max);
 }
-template<bool G>
+template<bool G, int kCalls>
 DORT_BD_FN bool bd_visible(const PtScene& sc, V3 a, float ea, V3 b, float eb) {
-  return lt_visible<G>(sc, a, ea, b, eb);
+  return lt_visible<G, kCalls>(sc, a, ea, b, eb);
 }
 template<bool G>
 DORT_BD_FN SurfaceHit bd_surface(const PtScene& sc, const Hit& h, V3 o, V3 d) {
@@ -295,7 +299,7 @@ DG_HD uint32_t bdpt_light_walk(const BdptCtx& c, uint32_t light_i, float pick, c
   float eps = ray.eps;
   for(uint32_t b = 0; b <= c.pp.max_depth && n < kBdptVerts; ++b) {
     ++rays;
-    Hit h = bd_trace<false, G>(sc, o, eps, d, INFINITY);
+    Hit h = bd_trace<false, G, 0>(sc, o, eps, d, INFINITY);
     if(h.prim == kMiss) { break; }
     SurfaceHit g = bd_surface<G>(sc, h, o, d);
     DevMaterial m = material_at(sc, g);
@@ -365,7 +369,7 @@ DG_HD uint32_t bdpt_camera_walk(const BdptCtx& c, float fx, float fy, const W& c
       scale = scale * (1.f / rr);
     }
     ++rays;
-    Hit h = bd_trace<false, G>(sc, o, eps, d, INFINITY);
+    Hit h = bd_trace<false, G, 0>(sc, o, eps, d, INFINITY);
     if(h.prim == kMiss) {
       // a virtual vertex on the background light picked by power
       // (background_light_distrib)
@@ -633,7 +637,7 @@ DG_HD bool bdpt_connect(const BdptCtx& c, const W& lw, const W& cw, const BdptSa
       if(We == 0.f) { return false; }
       if(sd.pick == 0.f) { return false; }
       ++rays;
-      Hit h = bd_trace<true, G>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
+      Hit h = bd_trace<true, G, 3 + int(CASE)>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
       if(h.prim != kMiss) { return false; }
       contrib = ls.L * (We / (cam_pdf * ls.pdf * sd.pick));
     } else {
@@ -670,7 +674,7 @@ DG_HD bool bdpt_connect(const BdptCtx& c, const W& lw, const W& cw, const BdptSa
       LightSample ls = bd_light_sample<G>(sc, l2, last_camera.p, last_camera.eps, rc.b, rc.c);
       if(is_black(ls.L) || ls.pdf == 0.f) { return false; }
       ++rays;
-      Hit h = bd_trace<true, G>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
+      Hit h = bd_trace<true, G, 3 + int(CASE)>(sc, ls.o, ls.tmin, ls.d, ls.tmax);
       if(h.prim != kMiss) { return false; }
       V3 bwo = normalize(cw.get(t - 2).p - last_camera.p);
       DevMaterial m = bvert_material(sc, last_camera);
@@ -711,7 +715,7 @@ DG_HD bool bdpt_connect(const BdptCtx& c, const W& lw, const W& cw, const BdptSa
       V3 f = bd_bsdf_eval<G>(m, bvert_frame(last_light), wi, wo, F_ALL);
       if(is_black(f)) { return false; }
       ++rays;
-      if(!bd_visible<G>(sc, last_light.p, last_light.eps, cam.p, 0.f)) { return false; }
+      if(!bd_visible<G, 3 + int(CASE)>(sc, last_light.p, last_light.eps, cam.p, 0.f)) { return false; }
       first_camera = bvert_empty();
       first_camera.p = cam.p;
       first_camera.fwd_pdf = cam.pdf;
@@ -728,7 +732,7 @@ DG_HD bool bdpt_connect(const BdptCtx& c, const W& lw, const W& cw, const BdptSa
     if constexpr(kAll || CASE == kBdCaseST) {
       const BVert last_light = lw.get(s - 1);
       ++rays;
-      if(!bd_visible<G>(sc, last_light.p, last_light.eps, last_camera.p, last_camera.eps)) {
+      if(!bd_visible<G, 3 + int(CASE)>(sc, last_light.p, last_light.eps, last_camera.p, last_camera.eps)) {
         return false;
       }
       V3 lwi = normalize(lw.get(s - 2).p - last_light.p);

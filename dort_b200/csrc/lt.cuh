@@ -352,13 +352,15 @@ DG_HD void lt_splat(float* film, const PtParams& pp, float fx, float fy, V3 c) {
 }
 
 // Unoccluded segment between two points (ShadowTest::init_point_point,
-// light.cpp:40-49): from a with epsilon ea to b with epsilon eb.
-template<bool G>
+// light.cpp:40-49): from a with epsilon ea to b with epsilon eb.  kCalls as in
+// path_trace (the light tracer's own three queries are inline: as calls 1.62
+// against 1.55 ms on a 256x256 Cornell box at 16 spp).
+template<bool G, int kCalls>
 DG_HD bool lt_visible(const PtScene& sc, V3 a, float ea, V3 b, float eb) {
   V3 d = b - a;
   float dist = length(d);
   if(!(dist > 0.f)) { return false; }
-  Hit h = scene_trace<true, G>(sc, a, ea, d * (1.f / dist), dist - eb);
+  Hit h = path_trace<true, G, kCalls>(sc, a, ea, d * (1.f / dist), dist - eb);
   return h.prim == kMiss;
 }
 
@@ -394,7 +396,7 @@ DG_HD uint32_t lt_path(const PtScene& sc, const PtParams& pp, uint32_t pixel, ui
           if(!is_black(lp.nn)) { c = c * fabsf(dot(lp.nn, normalize(to))); }
           if(!is_black(c)) {
             ++rays;
-            if(lt_visible<G>(sc, lp.p, lp.eps, cp, 0.f)) { lt_splat(film, pp, fx, fy, c); }
+            if(lt_visible<G, 0>(sc, lp.p, lp.eps, cp, 0.f)) { lt_splat(film, pp, fx, fy, c); }
           }
         }
       }
@@ -436,7 +438,7 @@ DG_HD uint32_t lt_path(const PtScene& sc, const PtParams& pp, uint32_t pixel, ui
           V3 c = thr * geom * f * (cam.We * fabsf(dot(g.n, cwo)) / (dist2 * cam.pdf));
           if(!is_black(c)) {
             ++rays;
-            if(lt_visible<G>(sc, g.p, g.eps, cam.p, 0.f)) { lt_splat(film, pp, cam.fx, cam.fy, c); }
+            if(lt_visible<G, 0>(sc, g.p, g.eps, cam.p, 0.f)) { lt_splat(film, pp, cam.fx, cam.fy, c); }
           }
         }
       }
