@@ -462,17 +462,17 @@ DG_HD const uint4* trav_next(TravState& s, const TraceScene& sc) {
 template<class Stack>
 DG_HD uint2 trav_enter(TravState& s, Stack& stack, uint32_t hits, uint32_t child_base,
                        uint32_t tri_base, uint32_t masks) {
+  // written as selects: as nested branches it cost 1.5 % of the ray cast
   const uint32_t inner = hits & masks & 0xffu;
-  if(inner) {
-    if(group_left(s)) {
-      // sp < kTraceStack: each push descends one level and the builder
-      // bounds the depth by kMaxWideDepth.
-      stack.push(s.sp++, s.group);
-    }
-    s.group = make_uint2(child_base, (masks << 8) | inner);
-  } else if(!group_left(s) && s.sp > 0) {
-    s.group = stack.pop(--s.sp);
-  }
+  const bool left = group_left(s);
+  // sp < kTraceStack: each push descends one level and the builder bounds the
+  // depth by kMaxWideDepth.
+  if(inner && left) { stack.push(s.sp, s.group); }
+  s.sp += (inner && left) ? 1 : 0;
+  const bool pop = !inner && !left && s.sp > 0;
+  s.sp -= pop ? 1 : 0;
+  if(inner) { s.group = make_uint2(child_base, (masks << 8) | inner); }
+  if(pop) { s.group = stack.pop(s.sp); }
   return make_uint2(tri_base, (masks & 0xffff0000u) | ((hits * 0x101u) & (masks >> 16)));
 }
 
