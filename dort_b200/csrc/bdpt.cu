@@ -45,14 +45,18 @@ constexpr uint32_t kBdptChunk = 1u << DORT_BDPT_CHUNK_LOG2;
 // Resident blocks per SM the register allocation must allow (Cornell
 // workload, A/B against the compiler's 104-128 registers): connection
 // kernels at 6 blocks +13 %, at 8 (64 registers, some spill) another +4 %;
-// walk kernels at 5 (96 registers) +8 %, and at 6 (80) once the traversal took
-// fewer registers (see bd_trace in bdpt.cuh).
+// walk kernels at 5 (96 registers) +8 %.  The fast instantiation (G = false)
+// fits 6 blocks (80 registers), since the traversal takes fewer registers.  The
+// general one at 6 spills: a 269x112 frame of shapes at 5 spp 526 us at
+// depth 2 and 1,114 at depth 8 against 507 and 1,076 with 5 (the Cornell box
+// with Phong surfaces 5.57 against 5.66 ms).
 #ifndef DORT_BDPT_CONNECT_MIN_BLOCKS
 #define DORT_BDPT_CONNECT_MIN_BLOCKS 8
 #endif
 #ifndef DORT_BDPT_WALK_MIN_BLOCKS
 #define DORT_BDPT_WALK_MIN_BLOCKS 6
 #endif
+constexpr int walk_blocks(bool general) { return general ? 5 : DORT_BDPT_WALK_MIN_BLOCKS; }
 
 // Connection slots of one sample: (s, t) with t >= 1 and s + t <= D =
 // max_depth + 2, numbered in the host loop's order (s outer, t inner); at
@@ -95,7 +99,7 @@ __device__ __forceinline__ uint32_t bd_case_count(uint32_t packed, uint32_t c) {
 // rec1 carries the pick, the light's index and the vertex count to the
 // camera walks.
 template<bool G>
-__global__ void __launch_bounds__(kBdptBlock, DORT_BDPT_WALK_MIN_BLOCKS)
+__global__ void __launch_bounds__(kBdptBlock, walk_blocks(G))
 bdpt_light_walks(PtScene sc, PtParams pp, uint64_t first, uint32_t count, BdptChunk ch,
                  unsigned long long* __restrict__ counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -125,7 +129,7 @@ bdpt_light_walks(PtScene sc, PtParams pp, uint64_t first, uint32_t count, BdptCh
 // The camera walks of a chunk, then each sample's connections: counted per
 // case, their slots marked for the gather, appended to the case lists.
 template<bool G>
-__global__ void __launch_bounds__(kBdptBlock, DORT_BDPT_WALK_MIN_BLOCKS)
+__global__ void __launch_bounds__(kBdptBlock, walk_blocks(G))
 bdpt_camera_walks(PtScene sc, PtParams pp, uint64_t first, uint32_t count, BdptChunk ch,
                   unsigned long long* __restrict__ counters) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

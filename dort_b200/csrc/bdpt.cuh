@@ -27,8 +27,8 @@ constexpr uint32_t kBdptVerts = 16;   // vertices per walk: max_depth <= 13
 // line.  Only the connections' ray queries are calls (path_trace): the kernels
 // are still bound by instruction fetch and 64 registers, and so the rest of a
 // connection keeps its registers around the traversal (256x256 Cornell box with
-// Phong surfaces at 16 spp, depth 8, together with 6 instead of 5 walk blocks per
-// SM: 5.92 -> 5.55 ms; with the walks' own queries as calls 6.02).
+// Phong surfaces at 16 spp, depth 8: 5.97 -> 5.66 ms; 269x112 frames of shapes
+// at 5 spp no slower; with the walks' own queries as calls 6.02).
 #ifdef DORT_BD_NOINLINE
 #define DORT_BD_FN __host__ __device__ __noinline__
 #else
