@@ -89,18 +89,18 @@ N_RAYS = 16 * 1024 * 1024
 # workload, from the ncu capture summarised in
 # profiles/raycast_kernel_1Mtri_16Mrays.md (dram__bytes_read.sum +
 # dram__bytes_write.sum); reported as the roofline's traffic.
-RAYCAST_TRAFFIC_BYTES = 800.7e6
+RAYCAST_TRAFFIC_BYTES = 815.3e6
 # The bound that applies to the ray cast beside the HBM roofline (whose
 # algorithmic bytes count the reference's binary-tree work, more than the
 # wide tree does, so its frac exceeds 1): issue slots.  Figures of one
-# launch under ncu --set full (profiles/raycast_kernel_1Mtri_16Mrays.md).
+# launch under ncu (profiles/raycast_kernel_1Mtri_16Mrays.md).
 RAYCAST_LIMITER = {
     "bound": "issue slots (divergent traversal)",
-    "source": "ncu --set full of one raycast_kernel launch, "
+    "source": "ncu capture of one raycast_kernel launch, "
               "profiles/raycast_kernel_1Mtri_16Mrays.md",
-    "issue_slots_busy": 0.739, "simt_efficiency": 11.6 / 32, "achieved_occupancy": 0.496,
-    "dram_throughput": 0.013,
-    "top_stall": "long_scoreboard, 3.85 cycles per issue",
+    "issue_slots_busy": 0.757, "simt_efficiency": 23.6 / 32, "achieved_occupancy": 0.495,
+    "l1_data_pipe": 0.669, "dram_throughput": 0.023,
+    "top_stall": "long_scoreboard, 3.04 cycles per issue",
 }
 WORKLOAD = "raycast: 1M random tris (SAH BVH), 16M rays (8M coherent pinhole 4096x2048 + 8M diffuse bounce), closest hit"
 
@@ -538,23 +538,24 @@ PT_WORKLOAD = ("pt1080p: wavefront path tracing 1920x1080, 256 spp, max depth 16
                "dielectric mix, procedural 1024x512 HDR sky")
 REF_SAMPLE_W, REF_SAMPLE_H = 480, 270
 # DRAM bytes (read + write) of one wf_extend launch over a full queue
-# (4,194,304 rays, waves 6-8 of the 16-spp frame), mean of three launches of
-# the ncu capture summarised in profiles/wf_extend_pt1080p.md: 777 MB, 185 B
+# (4,194,304 rays, a wave of the 16-spp frame), from
+# the ncu capture summarised in profiles/wf_extend_pt1080p.md: 613 MB, 146 B
 # per ray; reported as the roofline's traffic.
-EXTEND_TRAFFIC_BYTES = 730.4e6
+EXTEND_TRAFFIC_BYTES = 612.6e6
 EXTEND_TRAFFIC_RAYS = 4194304
 # The bound that applies to the extension stage beside the HBM roofline:
 # issue slots and latency.  Figures of one wf_extend launch under
-# ncu --set full (profiles/wf_extend_pt1080p.md): smsp__issue_active,
+# ncu (profiles/wf_extend_pt1080p.md): smsp__issue_active,
 # smsp__thread_inst_executed_per_inst_executed / 32, sm__warps_active,
 # lts__throughput and gpu__dram_throughput as fractions of their peaks.
 EXTEND_LIMITER = {
     "bound": "issue slots and node-fetch latency (divergent traversal)",
-    "source": "ncu --set full of one full-queue wf_extend launch, "
+    "source": "ncu capture of one full-queue wf_extend launch, "
               "profiles/wf_extend_pt1080p.md",
-    "issue_slots_busy": 0.668, "simt_efficiency": 11.92 / 32, "achieved_occupancy": 0.534,
-    "occupancy_limit": 0.5625, "l2_throughput": 0.178, "dram_throughput": 0.072,
-    "top_stall": "long_scoreboard (L1/L2 node and stack loads), 6.02 cycles per issue",
+    "issue_slots_busy": 0.655, "simt_efficiency": 24.23 / 32, "achieved_occupancy": 0.470,
+    "occupancy_limit": 0.5, "l1_data_pipe": 0.539, "l2_throughput": 0.196,
+    "dram_throughput": 0.095,
+    "top_stall": "long_scoreboard (L1/L2 node and stack loads), 5.25 cycles per issue",
 }
 
 _ref_worker_scene = None

@@ -10,7 +10,7 @@ namespace dort_gpu {
 
 // Device view of the ray-query part of a scene.
 struct TraceScene {
-  const uint4* nodes;   // 5 x uint4 per WideNode (bvh_build.h)
+  const uint4* nodes;   // 6 x uint4 per TraceNode (bvh_build.h)
   const float4* tris;   // 3 x float4 per LeafTri
   uint32_t node_count;
   uint32_t tri_count;

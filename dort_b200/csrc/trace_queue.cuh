@@ -34,6 +34,8 @@ __device__ __forceinline__ void prefetch_l2(const void* from, const void* to, ui
   if(p < to) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
 }
 
+// Neighbours (12 to 20, 6 to 10, 3 to 6) measured within 2 % on the soup's
+// camera and bounce rays; refilling at 8 idle lanes or more was slower.
 constexpr int kTriLanes = 16;
 constexpr int kMinLanes = 8;
 constexpr int kIdleLanes = 4;

@@ -73,18 +73,6 @@ constexpr uint32_t kMissQueue = 5;
 DG_HD uint32_t f2u(float f) { return DG_AS_UINT(f); }
 DG_HD float u2f(uint32_t u) { return DG_AS_FLOAT(u); }
 
-// Warp-aggregated append: returns this lane's index in the queue.
-__device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
-  uint32_t mask = __ballot_sync(0xffffffffu, want);
-  if(!want) { return 0; }
-  uint32_t lane = threadIdx.x & 31u;
-  uint32_t leader = __ffs(mask) - 1u;
-  uint32_t base = 0;
-  if(lane == leader) { base = atomicAdd(counter, __popc(mask)); }
-  base = __shfl_sync(mask, base, leader);
-  return base + __popc(mask & ((1u << lane) - 1u));
-}
-
 // Next 32 work items for this warp from a fetch cursor (lane 0 advances it).
 __device__ __forceinline__ uint32_t warp_fetch(uint32_t* cursor) {
   uint32_t base = 0;
@@ -596,8 +584,8 @@ __global__ void wf_classify(WfDev w) {
   }
 }
 
-// Register cap of the trace stages (extend, shadow, neeb): 8 blocks of 128
-// threads per SM.
+// Register cap of the trace stages (extend, light): 8 blocks of 128 threads
+// per SM.
 #ifndef DORT_TRACE_MAXNREG
 #define DORT_TRACE_MAXNREG 64
 #endif
