@@ -51,6 +51,7 @@ enum : uint32_t {
   C_LIVE = 6, C_WAVES = 7, C_ERROR = 8,
   C_F_EXT = 9, C_F_SHADE = 10, C_F_SH = 11, C_F_NB = 12,   // work-fetch cursors
   C_MORE = 13,      // whether another wave follows
+  C_NB_PAST = 14,   // this wave's BSDF-strategy rays past their light (not queued)
   C_KQ0 = 20,       // [20..25]: lengths of the shade queues by material kind
   C_NEXT_LO = 16,   // 64-bit next-sample counter at [16..17]
   C_RAYS_LO = 18,   // 64-bit ray counter at [18..19]
@@ -696,6 +697,7 @@ __device__ __forceinline__ void wave_begin(WfDev& w) {
   *ctr_at(w.ctr, C_FIN0 + cur) = 0u;
   *ctr_at(w.ctr, C_SHADOW) = 0u;
   *ctr_at(w.ctr, C_NEEB) = 0u;
+  *ctr_at(w.ctr, C_NB_PAST) = 0u;
   *ctr_at(w.ctr, C_F_SH) = 0u;
   *ctr_at(w.ctr, C_F_NB) = 0u;
   const uint64_t next = *reinterpret_cast<uint64_t*>(ctr_at(w.ctr, C_NEXT_LO));
@@ -714,7 +716,7 @@ __device__ __forceinline__ void wave_end(WfDev& w) {
   const uint32_t wave = wave_of(w);
   unsigned long long* rays = reinterpret_cast<unsigned long long*>(ctr_at(w.ctr, C_RAYS_LO));
   *rays += (unsigned long long)*ctr_at(w.ctr, C_ACT0 + (wave & 1u)) +
-           *ctr_at(w.ctr, C_SHADOW) + *ctr_at(w.ctr, C_NEEB);
+           *ctr_at(w.ctr, C_SHADOW) + *ctr_at(w.ctr, C_NEEB) + *ctr_at(w.ctr, C_NB_PAST);
   *ctr_at(w.ctr, C_F_EXT) = 0u;
   *ctr_at(w.ctr, C_F_SHADE) = 0u;
   for(uint32_t k = 0; k < kShadeQueues; ++k) { *ctr_at(w.ctr, C_KQ0 + k) = 0u; }
@@ -740,11 +742,42 @@ __global__ void DORT_TRACE_REGS wf_extend(J jobs, WfDev w) {
 //        ray escapes, and L and w depend on the direction alone, so it is an
 //        any-hit query with its contribution computed here;
 //   nb   the BSDF strategy towards an area light: closest hit, L and the MIS
-//        weight once the hit is known (NeebQueue).
+//        weight once the hit is known (NeebQueue);
+//   past the same where the ray passes the light's triangle by: nothing to
+//        trace, counted as a ray.
 struct NeeEntries {
-  bool sh, sh2, nb;
+  bool sh, sh2, nb, past;
   float4 sh_o, sh_d, sh_c, sh2_o, sh2_d, sh2_c, nb_o, nb_d, nb_f;
 };
+
+// Whether the ray passes a light's primitive by, so that its closest hit cannot
+// be that triangle: mt_fast as the traversal runs it on the same floats (the
+// primitive's; the light's own triangle may differ), with slack for the one sum
+// that the compiler may fuse differently there.  (Not for scenes traced with
+// the watertight test.)  Most BSDF-strategy rays do: of the Cornell box's 9.3M
+// in 64 spp the queue keeps so few that it takes 0.11 instead of 0.65 ms, and
+// shade, which does not write the others, 1.06 instead of 1.14.
+__device__ __forceinline__ bool passes_by(const PtScene& sc, uint32_t tri, V3 o, float t_min,
+                                          V3 d) {
+  const float4* r = sc.shade + 3 * size_t(tri);
+  const float4 p0 = __ldg(r), p1 = __ldg(r + 1), p2 = __ldg(r + 2);
+  const V3 e1 = v3(__fsub_rn(p1.x, p0.x), __fsub_rn(p1.y, p0.y), __fsub_rn(p1.z, p0.z));
+  const V3 e2 = v3(__fsub_rn(p2.x, p0.x), __fsub_rn(p2.y, p0.y), __fsub_rn(p2.z, p0.z));
+  const float s1x = DG_FMA(d.y, e2.z, -d.z * e2.y);
+  const float s1y = DG_FMA(d.z, e2.x, -d.x * e2.z);
+  const float s1z = DG_FMA(d.x, e2.y, -d.y * e2.x);
+  const float det = DG_FMA(s1x, e1.x, DG_FMA(s1y, e1.y, s1z * e1.z));
+  const float inv_det = DG_RCP_FAST(det);
+  const float sx = o.x - p0.x, sy = o.y - p0.y, sz = o.z - p0.z;
+  const float b1 = inv_det * DG_FMA(s1x, sx, DG_FMA(s1y, sy, s1z * sz));
+  const float s2x = DG_FMA(sy, e1.z, -sz * e1.y);
+  const float s2y = DG_FMA(sz, e1.x, -sx * e1.z);
+  const float s2z = DG_FMA(sx, e1.y, -sy * e1.x);
+  const float b2 = inv_det * DG_FMA(s2x, d.x, DG_FMA(s2y, d.y, s2z * d.z));
+  const float t = inv_det * DG_FMA(s2x, e2.x, DG_FMA(s2y, e2.y, s2z * e2.z));
+  const float slack = 1e-5f;
+  return b1 < -slack || b2 < -slack || b1 + b2 > 1.f + slack || t < t_min * (1.f - slack);
+}
 
 template<bool G, bool ADJ = false>
 __device__ __forceinline__ void nee_entries(const PtScene& sc, const PtParams& pp, uint32_t li,
@@ -753,7 +786,7 @@ __device__ __forceinline__ void nee_entries(const PtScene& sc, const PtParams& p
                                             float vb, float cb, float ul, float vl,
                                             NeeEntries& e) {
   const uint32_t req_nd = F_ALL & ~F_DELTA;
-  e.sh = e.sh2 = e.nb = false;
+  e.sh = e.sh2 = e.nb = e.past = false;
   const DevLight& l = sc.lights[li];
   // the BSDF strategy only for area and background lights
   // (path_renderer.cpp:138-140)
@@ -762,10 +795,12 @@ __device__ __forceinline__ void nee_entries(const PtScene& sc, const PtParams& p
   if(use_bsdf) {
     BsdfSample bs = bsdf_sample<G>(mt, g.frame, wo, req_nd, ub, vb, cb);
     if(!(bs.pdf == 0.f || is_black(bs.f))) {
+      e.past = l.kind == LIGHT_TRI && !(G && sc.trace.watertight) &&
+               passes_by(sc, l.tri, g.p, g.eps, bs.w);
       // contribution = f * L * (w |n.wi| / pdf) * thr / light_pick_pdf
       V3 fac = thr * (bs.f * (fabsf(dot(g.n, bs.w)) / bs.pdf)) * inv_lpdf;
       if(light_is_area(l)) {
-        e.nb = true;
+        e.nb = !e.past;
         e.nb_o = make_float4(g.p.x, g.p.y, g.p.z, g.eps);
         e.nb_d = make_float4(bs.w.x, bs.w.y, bs.w.z, bs.pdf);
         e.nb_f = make_float4(fac.x, fac.y, fac.z, u2f(li | (use_light ? 0x80000000u : 0u)));
@@ -852,6 +887,7 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
   }
   const uint32_t req_nd = F_ALL & ~F_DELTA;
   const uint32_t lane = threadIdx.x & 31u;
+  uint32_t past = 0;
   for(;;) {
     uint32_t base = warp_fetch(ctr_at(w.ctr, C_F_SHADE));
     if(base >= n) { break; }
@@ -859,7 +895,7 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
     bool valid = i < n;
     bool cont = false, done = false;
     NeeEntries nee;
-    nee.sh = nee.sh2 = nee.nb = false;
+    nee.sh = nee.sh2 = nee.nb = nee.past = false;
     uint32_t slot = 0;
     if(valid) {
       // index i of the concatenated shade queues
@@ -936,6 +972,7 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
               nee_entries<J::kGeneral, J::kAdjoint>(sc, pp, li, 1.f, g, mt, wo, thr, a.a, a.b,
                                                     a.c, b.a, b.b, e);
               push_entries(w, slot, e);
+              past += e.past ? 1u : 0u;
             }
           } else {
             uint32_t li = distrib_sample(sc.light_cdf, sc.light_count + 1, r0.a);
@@ -981,6 +1018,7 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
     }
     (void)cont;
     (void)done;
+    past += nee.past ? 1u : 0u;
     // the entries of the shadow queue (both strategies) and of the BSDF-strategy
     // queue: one atomic a queue, both at once
     const uint32_t m1 = __ballot_sync(0xffffffffu, nee.sh);
@@ -1017,6 +1055,8 @@ __global__ void DORT_SHADE_REGS wf_shade(J jobs, WfDev w, WfLoop loop) {
       w.nb_f[ni] = nee.nb_f;
     }
   }
+  past = __reduce_add_sync(0xffffffffu, past);
+  if(lane == 0 && past) { atomicAdd(ctr_at(w.ctr, C_NB_PAST), past); }
 }
 
 // A shadow-queue entry that nothing blocks: its contribution joins its path's
@@ -1695,9 +1735,9 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
   SingleJob<G> jobs{s->pt, pp};
   WfGrids g = wf_grids<SingleJob<G>>(tn);
   wf->dev.sorted = tn.sort;
-  // more[0]: loop flag; more[1..6]: the counters C_ACT0 .. C_NEEB of the wave
+  // more[0]: loop flag; more[1..]: the counters C_ACT0 .. C_NB_PAST of the wave
   uint32_t* more = nullptr;
-  DG_CUDA(host_pinned_alloc(&more, 8 * sizeof(uint32_t)));
+  DG_CUDA(host_pinned_alloc(&more, 16 * sizeof(uint32_t)));
   cudaEvent_t ev[6];
   for(auto& e : ev) { cudaEventCreate(&e); }
   for(int k = 0; k < 6; ++k) { ms[k] = 0.0; }
@@ -1718,7 +1758,7 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
     wf_launch_light<SingleJob<G>>(jobs, wf->dev, tn, g, LIGHT_NEEB | LIGHT_END, st);
     cudaEventRecord(ev[5], st);
     cudaMemcpy2DAsync(more + 1, sizeof(uint32_t), wf->dev.ctr, kCtrStride * sizeof(uint32_t),
-                      sizeof(uint32_t), C_NEEB + 1, cudaMemcpyDeviceToHost, st);
+                      sizeof(uint32_t), C_NB_PAST + 1, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(more, ctr_at(wf->dev.ctr, C_MORE), sizeof(uint32_t), cudaMemcpyDeviceToHost,
                     st);
     ok = cudaStreamSynchronize(st) == cudaSuccess;
@@ -1730,7 +1770,7 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
     if(ok) {
       stage_rays[0] += double(more[1 + C_ACT0 + (wave & 1u)]);
       stage_rays[1] += double(more[1 + C_SHADOW]);
-      stage_rays[2] += double(more[1 + C_NEEB]);
+      stage_rays[2] += double(more[1 + C_NEEB]) + double(more[1 + C_NB_PAST]);
     }
     if(!*more) { break; }
   }
