@@ -13,10 +13,10 @@
 //           their MIS weight
 //
 // The waves run inside one CUDA graph per frame: a conditional while node
-// whose body holds the four kernels, so the host launches a frame once.  The
-// loop condition is known after regen (extend notes it, shade sets it); the queue
-// counters are reset by the next kernel that does not use them (wave_begin,
-// wave_end).
+// whose body holds the four kernels (five with deterministic sums), so the host
+// launches a frame once.  The loop condition is known after regen (extend notes
+// it, shade sets it); the queue counters are reset by the next kernel that does
+// not use them (wave_begin, wave_end).
 // Queues are compacted with warp ballots (one atomic per warp).  Every kernel
 // is a grid-stride loop over a count it reads from device memory, so the
 // graph's launch shapes are fixed.
@@ -1284,9 +1284,9 @@ struct NeebQueue {
 };
 
 // The direct lighting of a wave: its shadow queue, its BSDF-strategy queue,
-// and the end of the wave (`parts`; one launch does all three, the stage
-// timing one after the other).  One kernel, so that a warp goes on with the
-// second queue while others finish the first.
+// and the end of the wave (`parts`).  One launch does all three, so that a warp
+// goes on with the second queue while others finish the first; frames with
+// deterministic sums and the stage timing run one queue after the other.
 enum : uint32_t { LIGHT_SHADOW = 1, LIGHT_NEEB = 2, LIGHT_END = 4, LIGHT_ALL = 7 };
 
 template<class J, bool STAGED>
@@ -1534,7 +1534,15 @@ static void wf_launch_wave(const J& jobs, WfDev& dev, const WfTuning& tn, const 
   wf_regen<J><<<g.regen, kRegenBlock, 0, st>>>(jobs, dev);
   wf_launch_extend<J>(jobs, dev, tn, g, st);
   wf_shade<J><<<g.sha, g.b_sha, 0, st>>>(jobs, dev, loop);
-  wf_launch_light<J>(jobs, dev, tn, g, LIGHT_ALL, st);
+  if(tn.deterministic) {
+    // a path may have an entry in each of the light stage's queues, and the
+    // order in which the two are added to its sum shows in the last bits: the
+    // second queue starts when the first is done
+    wf_launch_light<J>(jobs, dev, tn, g, LIGHT_SHADOW, st);
+    wf_launch_light<J>(jobs, dev, tn, g, LIGHT_NEEB | LIGHT_END, st);
+  } else {
+    wf_launch_light<J>(jobs, dev, tn, g, LIGHT_ALL, st);
+  }
 }
 
 template<class J>
