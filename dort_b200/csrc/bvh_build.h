@@ -18,11 +18,12 @@
 //     uint8_t  qlo[3][8], qhi[3][8]   quantized child boxes
 //   TraceNode: the same as the device traverses it (three 32-byte loads)
 //
-// Child boxes are quantized outward with a margin that covers the rounding of
-// the device slab test and of the triangle test (bvh_wide.h), so that no
-// child that contains a hit is culled.  (One grid step of margin on a
-// power-of-two grid, the form before, made the boxes larger: 4M camera rays on
-// the 1M-triangle soup 1.59 against 1.51 ms, 3M shadow rays on a 250k-triangle
+// Child boxes are quantized outward with 1/32 of a grid step to spare, which
+// covers the rounding of the device slab test's decoding; the triangle test's
+// own rounding grows with the distance from the ray and is covered there
+// (trace.cuh, DORT_RAY_MARGIN).  (One grid step of margin on a power-of-two
+// grid, the form before, made the boxes larger: 4M camera rays on the
+// 1M-triangle soup 1.59 against 1.51 ms, 3M shadow rays on a 250k-triangle
 // sphere 0.90 against 0.85 ms.)
 //
 //   Triangle (48 bytes = 3 x float4, leaf order):

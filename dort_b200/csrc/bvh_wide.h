@@ -121,13 +121,12 @@ BW_HD void assign_slots(const A& acc, const uint32_t* cands, uint32_t n, float n
 }
 
 // Picks the quantization grid of one axis: origin p, step s, and for every
-// child planes that enclose it with `margin` to spare (and 1/32 of a step, for
-// the rounding of the device's decoding).  253 steps cover the extent.
-// Returns false if no step fits.
-BW_HD bool quantize_axis(float node_lo, float node_hi, double margin, const float* clo,
-                         const float* chi, int n, float& p_out, float& s_out, uint8_t* qlo,
-                         uint8_t* qhi) {
-  const double lo = BW_SUB(double(node_lo), margin), hi = BW_ADD(double(node_hi), margin);
+// child planes that enclose it with 1/32 of a step to spare, for the rounding
+// of the device's decoding.  253 steps cover the extent.  Returns false if no
+// step fits.
+BW_HD bool quantize_axis(float node_lo, float node_hi, const float* clo, const float* chi, int n,
+                         float& p_out, float& s_out, uint8_t* qlo, uint8_t* qhi) {
+  const double lo = node_lo, hi = node_hi;
   const double mag = fmax(fabs(lo), fabs(hi));
   const double min_step = fmax(BW_MUL(mag, ldexp(1.0, -20)), ldexp(1.0, -100));
   double step = fmax(BW_SUB(hi, lo) / 253.0, min_step);
@@ -136,8 +135,8 @@ BW_HD bool quantize_axis(float node_lo, float node_hi, double margin, const floa
     if(double(sf) < step) { sf = nextafterf(sf, INFINITY); }
     const double s = double(sf);
     if(!(s <= 1e30)) { return false; }
-    const double spare = BW_ADD(margin, BW_MUL(s, 0.03125));
-    const double pd = BW_SUB(double(node_lo), spare);
+    const double spare = BW_MUL(s, 0.03125);
+    const double pd = BW_SUB(lo, spare);
     float pf = float(pd);
     if(double(pf) > pd) { pf = nextafterf(pf, -INFINITY); }
     const double p = double(pf);
@@ -161,7 +160,7 @@ BW_HD bool quantize_axis(float node_lo, float node_hi, double margin, const floa
 }
 
 // Quantizes the 8 slot boxes of a node (empty slots: cand_in_slot < 0) into
-// `node` (p, e, qlo, qhi); empty slots get an inverted box.
+// `node` (p, s, qlo, qhi); empty slots get an inverted box.
 template<class A>
 BW_HD bool quantize_node(const A& acc, const uint32_t* cands, const int cand_in_slot[8],
                          const float nlo[3], const float nhi[3], WideNode& node) {
@@ -173,15 +172,9 @@ BW_HD bool quantize_node(const A& acc, const uint32_t* cands, const int cand_in_
       chi[a][s] = c >= 0 ? acc.hi(cands[c])[a] : nlo[a];
     }
   }
-  // The boxes' margin: 2^-14 of the node's largest coordinate, for the rounding
-  // of the triangle test (a few 2^-24 of the distance to the triangle), which
-  // may report hits that miss the exact box by that.
-  double mag = 0.0;
-  for(int a = 0; a < 3; ++a) { mag = fmax(mag, fmax(fabs(double(nlo[a])), fabs(double(nhi[a])))); }
-  const double margin = BW_MUL(mag, ldexp(1.0, -14));
   for(int a = 0; a < 3; ++a) {
-    if(!quantize_axis(nlo[a], nhi[a], margin, clo[a], chi[a], 8, node.p[a], node.s[a],
-                      node.qlo[a], node.qhi[a])) {
+    if(!quantize_axis(nlo[a], nhi[a], clo[a], chi[a], 8, node.p[a], node.s[a], node.qlo[a],
+                      node.qhi[a])) {
       return false;
     }
   }

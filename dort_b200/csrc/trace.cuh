@@ -9,10 +9,13 @@
 // Traversal: node groups (base index, internal-slot mask << 8 | child-hit
 // bits) on a per-thread stack; child slots are visited in an order fixed by
 // the ray octant (slot bit index XOR octant), so no per-node sort is needed.
-// Child boxes are tested with fused multiply-adds on the quantized planes and
-// a relative widening that covers the rounding of that arithmetic
-// (DORT_SLAB_FAR_WIDEN); together with the one-step quantization margin the
-// test never culls a box containing a hit.
+// Child boxes are tested with fused multiply-adds on the quantized planes.  The
+// quantization's 1/32 step covers the rounding of the planes' decoding, a
+// relative widening (DORT_SLAB_FAR_WIDEN) that of the distances, and a margin
+// that grows with the distance from the ray's origin to the node
+// (DORT_RAY_MARGIN) that of the triangle test.  That margin is wide enough for
+// triangles of ordinary shape; a sliver's test may be off by more, so that a
+// hit that it reports beside its box may be culled.
 //
 // Triangle test: the reference's Moller-Trumbore operations in the
 // reference's order with explicit round-to-nearest intrinsics (no fused
@@ -264,6 +267,56 @@ DG_HD void load_32(const uint4* p, uint32_t v[8]) {
 
 constexpr uint32_t kNodeWords = 6;   // uint4 words per TraceNode
 
+// The box test's margin for the triangle test's rounding.  A triangle test sees
+// a triangle at distance D through coordinates rounded to about 2^-24 D, so it
+// may report a hit where the ray passes the triangle, and with it its box, by a
+// small multiple of that: a few units for a triangle about as high as wide,
+// times its aspect and the ray's slant to it.  The margin is 2^-16 (256 units)
+// of the largest coordinate difference between the ray's origin and the node.
+// It is the ray's and not the boxes', since the error is: a margin in the boxes
+// of 2^-14 of the node's largest coordinate lost hits of meshes at the
+// coordinate origin (a 0.04 wide one seen from 10 and more of its widths away)
+// and made the nodes of small meshes far from it overlap (the same mesh at
+// (100, 0, 50): 129 node visits a ray instead of 7).  2^-18 and 2^-17 measured
+// no faster (1M-triangle soup, 16.8M rays: 7.32 ms with each; without the
+// term and with the margin in the boxes 7.23); of 900k rays aimed at edges from
+// 1,000 mesh sizes away they lost 138 and 68, this one none.
+#define DORT_RAY_MARGIN 1.52587890625e-5f
+
+// A ray's view of a node's quantization grid.  The distance of plane q on an
+// axis is t = (p + s q - o) i; a near plane's, less the margin, is
+// (32768 + q) a + b, a far plane's, plus the margin, (65536 + q) a + c.  (The
+// rounding of b and c is below a / 128, of the 1/32 step's a / 32.)
+struct NodeSlabs {
+  float ax, ay, az, bx, by, bz, cx, cy, cz;
+};
+DG_HD NodeSlabs node_slabs(const uint32_t n0[8], float ox, float oy, float oz, float ix, float iy,
+                           float iz) {
+  NodeSlabs f;
+  const float px = DG_AS_FLOAT(n0[0]) - ox, py = DG_AS_FLOAT(n0[1]) - oy,
+              pz = DG_AS_FLOAT(n0[2]) - oz;
+  const float m = DORT_RAY_MARGIN * DG_MAX3(fabsf(px), fabsf(py), fabsf(pz));
+  const float wx = m * fabsf(ix), wy = m * fabsf(iy), wz = m * fabsf(iz);
+  f.ax = DG_AS_FLOAT(n0[3]) * ix;
+  f.ay = DG_AS_FLOAT(n0[4]) * iy;
+  f.az = DG_AS_FLOAT(n0[5]) * iz;
+  f.bx = DG_FMA(-32768.f, f.ax, DG_FMA(px, ix, -wx));
+  f.by = DG_FMA(-32768.f, f.ay, DG_FMA(py, iy, -wy));
+  f.bz = DG_FMA(-32768.f, f.az, DG_FMA(pz, iz, -wz));
+  f.cx = DG_FMA(-65536.f, f.ax, DG_FMA(px, ix, wx));
+  f.cy = DG_FMA(-65536.f, f.ay, DG_FMA(py, iy, wy));
+  f.cz = DG_FMA(-65536.f, f.az, DG_FMA(pz, iz, wz));
+  return f;
+}
+
+// Whether a ray's [t_min, t_max] meets a box of near distance tn and far
+// distance tf, as a sign bit (set: it does not).  t_far_max = t_max widened.
+DG_HD float slab_sign(float tn, float tf, float t_min, float t_far_max) {
+  tf = DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, tf);
+  // tn <= tf, t_min <= tf and tn <= t_far_max: no difference is negative
+  return DG_MIN3(tf - tn, tf - t_min, t_far_max - tn);
+}
+
 // Tests the 8 child boxes of one node (TraceNode, as three 32-byte loads):
 // bit s of the result is set when the ray's [t_min, t_max] meets slot s's
 // box (t_far_max = t_max widened).  Empty slots have no bit in either mask of
@@ -280,15 +333,7 @@ constexpr uint32_t kNodeWords = 6;   // uint4 words per TraceNode
 DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
                          float ox, float oy, float oz, float ix, float iy, float iz,
                          float t_min, float t_far_max) {
-  // t of plane q on an axis: (p + s q - o) i = (32768 + q) a + b = (65536 + q) a + c
-  // (b and c are off by less than a / 128, of the margin's a)
-  const float ax = DG_AS_FLOAT(n0[3]) * ix, ay = DG_AS_FLOAT(n0[4]) * iy,
-              az = DG_AS_FLOAT(n0[5]) * iz;
-  const float bx = DG_FMA(-32768.f, ax, (DG_AS_FLOAT(n0[0]) - ox) * ix);
-  const float by = DG_FMA(-32768.f, ay, (DG_AS_FLOAT(n0[1]) - oy) * iy);
-  const float bz = DG_FMA(-32768.f, az, (DG_AS_FLOAT(n0[2]) - oz) * iz);
-  const float cx = DG_FMA(-32768.f, ax, bx), cy = DG_FMA(-32768.f, ay, by),
-              cz = DG_FMA(-32768.f, az, bz);
+  const NodeSlabs f = node_slabs(n0, ox, oy, oz, ix, iy, iz);
   // near / far plane bytes per axis, by direction sign
   const bool nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
   const uint32_t near_x[2] = { nx ? n1[4] : n1[2], nx ? n1[5] : n1[3] };
@@ -302,41 +347,35 @@ DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint3
 #pragma unroll
   for(int s = 7; s >= 0; --s) {
     const int h = s >> 2, j = s & 3;
-    const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(near_x[h], one, j), ax, bx),
-                             DG_FMA(DG_BYTE_FLOAT(near_y[h], one, j), ay, by),
-                             DG_FMA(DG_BYTE_FLOAT(near_z[h], one, j), az, bz));
-    float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT_DP(far_x[h], j), ax, cx),
-                       DG_FMA(DG_BYTE_FLOAT_DP(far_y[h], j), ay, cy),
-                       DG_FMA(DG_BYTE_FLOAT_DP(far_z[h], j), az, cz));
-    tf = DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, tf);
-    // tn <= tf, t_min <= tf and tn <= t_far_max: no difference is negative
-    miss = DG_PUSH_SIGN(miss, DG_MIN3(tf - tn, tf - t_min, t_far_max - tn));
+    const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(near_x[h], one, j), f.ax, f.bx),
+                             DG_FMA(DG_BYTE_FLOAT(near_y[h], one, j), f.ay, f.by),
+                             DG_FMA(DG_BYTE_FLOAT(near_z[h], one, j), f.az, f.bz));
+    const float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT_DP(far_x[h], j), f.ax, f.cx),
+                             DG_FMA(DG_BYTE_FLOAT_DP(far_y[h], j), f.ay, f.cy),
+                             DG_FMA(DG_BYTE_FLOAT_DP(far_z[h], j), f.az, f.cz));
+    miss = DG_PUSH_SIGN(miss, slab_sign(tn, tf, t_min, t_far_max));
   }
   return ~miss & 0xffu;
 }
 
-// The same test for slot `slot` alone (a lane per slot, trace_wide).
+// The same test, operation for operation, for slot `slot` alone (a lane per
+// slot, trace_wide).
 DG_HD bool slot_hit(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
                     uint32_t slot, float ox, float oy, float oz, float ix, float iy, float iz,
                     float t_min, float t_far_max) {
-  const float ax = DG_AS_FLOAT(n0[3]) * ix, ay = DG_AS_FLOAT(n0[4]) * iy,
-              az = DG_AS_FLOAT(n0[5]) * iz;
-  const float bx = DG_FMA(-32768.f, ax, (DG_AS_FLOAT(n0[0]) - ox) * ix);
-  const float by = DG_FMA(-32768.f, ay, (DG_AS_FLOAT(n0[1]) - oy) * iy);
-  const float bz = DG_FMA(-32768.f, az, (DG_AS_FLOAT(n0[2]) - oz) * iz);
+  const NodeSlabs f = node_slabs(n0, ox, oy, oz, ix, iy, iz);
   const bool h = slot >= 4u, nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
   const uint32_t lo_x = h ? n1[3] : n1[2], hi_x = h ? n1[5] : n1[4];
   const uint32_t lo_y = h ? n1[7] : n1[6], hi_y = h ? n2[1] : n2[0];
   const uint32_t lo_z = h ? n2[3] : n2[2], hi_z = h ? n2[5] : n2[4];
   const uint32_t one = n1[1], j = slot & 3u;
-  const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(nx ? hi_x : lo_x, one, j), ax, bx),
-                           DG_FMA(DG_BYTE_FLOAT(ny ? hi_y : lo_y, one, j), ay, by),
-                           DG_FMA(DG_BYTE_FLOAT(nz ? hi_z : lo_z, one, j), az, bz));
-  float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT(nx ? lo_x : hi_x, one, j), ax, bx),
-                     DG_FMA(DG_BYTE_FLOAT(ny ? lo_y : hi_y, one, j), ay, by),
-                     DG_FMA(DG_BYTE_FLOAT(nz ? lo_z : hi_z, one, j), az, bz));
-  tf = DG_FMA(fabsf(tf), DORT_SLAB_FAR_WIDEN, tf);
-  return (DG_AS_UINT(DG_MIN3(tf - tn, tf - t_min, t_far_max - tn)) >> 31) == 0u;
+  const float tn = DG_MAX3(DG_FMA(DG_BYTE_FLOAT(nx ? hi_x : lo_x, one, j), f.ax, f.bx),
+                           DG_FMA(DG_BYTE_FLOAT(ny ? hi_y : lo_y, one, j), f.ay, f.by),
+                           DG_FMA(DG_BYTE_FLOAT(nz ? hi_z : lo_z, one, j), f.az, f.bz));
+  const float tf = DG_MIN3(DG_FMA(DG_BYTE_FLOAT_DP(nx ? lo_x : hi_x, j), f.ax, f.cx),
+                           DG_FMA(DG_BYTE_FLOAT_DP(ny ? lo_y : hi_y, j), f.ay, f.cy),
+                           DG_FMA(DG_BYTE_FLOAT_DP(nz ? lo_z : hi_z, j), f.az, f.cz));
+  return (DG_AS_UINT(slab_sign(tn, tf, t_min, t_far_max)) >> 31) == 0u;
 }
 
 // Traversal state of one ray.  trav_node visits one node, trav_tri tests one
