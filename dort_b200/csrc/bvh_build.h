@@ -53,6 +53,9 @@ struct WideNode {
   uint8_t qhi[3][8];
 };
 
+// Limit of the box test's margin in the largest of a node's steps.
+constexpr float kMarginSteps = 4.f;
+
 // The same node as the device traverses it.  96 bytes = three 32-byte loads.
 struct alignas(32) TraceNode {
   float p[3];            // origin of the quantization grid
@@ -62,7 +65,8 @@ struct alignas(32) TraceNode {
   uint32_t masks;        // bits 0..7: imask; bit 16 + 8 k + s: slot s is a leaf of more than k triangles
   uint32_t byte_one;     // 32768.f: a plane byte in its second byte makes the float 32768 + byte
   uint32_t q[3][2][2];   // [axis][0: lo, 1: hi][slots 0..3, 4..7]: child planes, a byte per slot
-  uint32_t pad1[2];
+  float margin_max;      // upper limit of the box test's margin (trace.cuh): kMarginSteps steps
+  uint32_t pad;
 };
 static_assert(sizeof(TraceNode) == 96, "TraceNode must be 96 bytes");
 

@@ -209,7 +209,8 @@ BW_HD void pack_trace_node(const WideNode& n, TraceNode& t) {
     if(n.meta[k] > 1) { t.masks |= 1u << (24 + k); }
   }
   t.byte_one = 0x47000000u;
-  t.pad1[0] = t.pad1[1] = 0;
+  t.margin_max = kMarginSteps * fmaxf(n.s[0], fmaxf(n.s[1], n.s[2]));
+  t.pad = 0;
 }
 
 }  // namespace dort_gpu

@@ -270,42 +270,47 @@ constexpr uint32_t kNodeWords = 6;   // uint4 words per TraceNode
 // The box test's margin for the triangle test's rounding.  A triangle test sees
 // a triangle at distance D through coordinates rounded to about 2^-24 D, so it
 // may report a hit where the ray passes the triangle, and with it its box, by a
-// small multiple of that: a few units for a triangle about as high as wide,
-// times its aspect and the ray's slant to it.  The margin is 2^-16 (256 units)
-// of the largest coordinate difference between the ray's origin and the node.
-// It is the ray's and not the boxes', since the error is: a margin in the boxes
-// of 2^-14 of the node's largest coordinate lost hits of meshes at the
+// small multiple of that: at most some 20 units for a triangle about as high as
+// wide, times its aspect and the ray's slant to it.  The margin is 2^-16 (256
+// units) of the largest coordinate difference between the ray's origin and the
+// node, but at most four of the node's largest grid steps (TraceNode::
+// margin_max).  Without that limit rays from far away visit whole trees: a grid
+// of 500 x 500 quads took 162 node visits a ray from 1,000 of its widths away
+// and 5,700 from 10,000, against 14 and 72 with it (2 steps: 12 and 69; 8: 18
+// and 80).  It only counts where 2^-24 D nears the size of a triangle.
+// The margin is the ray's and not the boxes', since the error is: a margin in
+// the boxes of 2^-14 of the node's largest coordinate lost hits of meshes at the
 // coordinate origin (a 0.04 wide one seen from 10 and more of its widths away)
 // and made the nodes of small meshes far from it overlap (the same mesh at
-// (100, 0, 50): 129 node visits a ray instead of 7).  2^-18 and 2^-17 measured
-// no faster (1M-triangle soup, 16.8M rays: 7.32 ms with each; without the
-// term and with the margin in the boxes 7.23); of 900k rays aimed at edges from
-// 1,000 mesh sizes away they lost 138 and 68, this one none.
+// (100, 0, 50): 129 node visits a ray instead of 7).
 #define DORT_RAY_MARGIN 1.52587890625e-5f
 
 // A ray's view of a node's quantization grid.  The distance of plane q on an
 // axis is t = (p + s q - o) i; a near plane's, less the margin, is
 // (32768 + q) a + b, a far plane's, plus the margin, (65536 + q) a + c.  (The
-// rounding of b and c is below a / 128, of the 1/32 step's a / 32.)
+// rounding of b and c is below a / 100, of the 1/32 step's a / 32.)
 struct NodeSlabs {
   float ax, ay, az, bx, by, bz, cx, cy, cz;
 };
-DG_HD NodeSlabs node_slabs(const uint32_t n0[8], float ox, float oy, float oz, float ix, float iy,
-                           float iz) {
+DG_HD NodeSlabs node_slabs(const uint32_t n0[8], float margin_max, float ox, float oy, float oz,
+                           float ix, float iy, float iz) {
   NodeSlabs f;
   const float px = DG_AS_FLOAT(n0[0]) - ox, py = DG_AS_FLOAT(n0[1]) - oy,
               pz = DG_AS_FLOAT(n0[2]) - oz;
-  const float m = DORT_RAY_MARGIN * DG_MAX3(fabsf(px), fabsf(py), fabsf(pz));
-  const float wx = m * fabsf(ix), wy = m * fabsf(iy), wz = m * fabsf(iz);
+  const float m = fminf(DORT_RAY_MARGIN * DG_MAX3(fabsf(px), fabsf(py), fabsf(pz)), margin_max);
   f.ax = DG_AS_FLOAT(n0[3]) * ix;
   f.ay = DG_AS_FLOAT(n0[4]) * iy;
   f.az = DG_AS_FLOAT(n0[5]) * iz;
-  f.bx = DG_FMA(-32768.f, f.ax, DG_FMA(px, ix, -wx));
-  f.by = DG_FMA(-32768.f, f.ay, DG_FMA(py, iy, -wy));
-  f.bz = DG_FMA(-32768.f, f.az, DG_FMA(pz, iz, -wz));
-  f.cx = DG_FMA(-65536.f, f.ax, DG_FMA(px, ix, wx));
-  f.cy = DG_FMA(-65536.f, f.ay, DG_FMA(py, iy, wy));
-  f.cz = DG_FMA(-65536.f, f.az, DG_FMA(pz, iz, wz));
+  // the margin comes last: a lone ray waits for the chain that leads to it
+  f.bx = DG_FMA(-32768.f, f.ax, px * ix);
+  f.by = DG_FMA(-32768.f, f.ay, py * iy);
+  f.bz = DG_FMA(-32768.f, f.az, pz * iz);
+  f.cx = DG_FMA(m, fabsf(ix), DG_FMA(-32768.f, f.ax, f.bx));
+  f.cy = DG_FMA(m, fabsf(iy), DG_FMA(-32768.f, f.ay, f.by));
+  f.cz = DG_FMA(m, fabsf(iz), DG_FMA(-32768.f, f.az, f.bz));
+  f.bx = DG_FMA(-m, fabsf(ix), f.bx);
+  f.by = DG_FMA(-m, fabsf(iy), f.by);
+  f.bz = DG_FMA(-m, fabsf(iz), f.bz);
   return f;
 }
 
@@ -333,7 +338,7 @@ DG_HD float slab_sign(float tn, float tf, float t_min, float t_far_max) {
 DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
                          float ox, float oy, float oz, float ix, float iy, float iz,
                          float t_min, float t_far_max) {
-  const NodeSlabs f = node_slabs(n0, ox, oy, oz, ix, iy, iz);
+  const NodeSlabs f = node_slabs(n0, DG_AS_FLOAT(n2[6]), ox, oy, oz, ix, iy, iz);
   // near / far plane bytes per axis, by direction sign
   const bool nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
   const uint32_t near_x[2] = { nx ? n1[4] : n1[2], nx ? n1[5] : n1[3] };
@@ -363,7 +368,7 @@ DG_HD uint32_t node_hits(const uint32_t n0[8], const uint32_t n1[8], const uint3
 DG_HD bool slot_hit(const uint32_t n0[8], const uint32_t n1[8], const uint32_t n2[8],
                     uint32_t slot, float ox, float oy, float oz, float ix, float iy, float iz,
                     float t_min, float t_far_max) {
-  const NodeSlabs f = node_slabs(n0, ox, oy, oz, ix, iy, iz);
+  const NodeSlabs f = node_slabs(n0, DG_AS_FLOAT(n2[6]), ox, oy, oz, ix, iy, iz);
   const bool h = slot >= 4u, nx = ix < 0.f, ny = iy < 0.f, nz = iz < 0.f;
   const uint32_t lo_x = h ? n1[3] : n1[2], hi_x = h ? n1[5] : n1[4];
   const uint32_t lo_y = h ? n1[7] : n1[6], hi_y = h ? n2[1] : n2[0];

@@ -8,6 +8,8 @@ box around it, by its own rounding, which grows with the distance.
 Not compared: rays within 0.02 of parallel to the triangle that either side
 found.  Their distance is off by 50 times the rounding and more, so the order
 of two triangles' distances is not defined in 32 bits."""
+import time
+
 import numpy as np
 import pytest
 
@@ -90,6 +92,50 @@ def test_no_hit_is_culled(kind, where, sizes, count):
     _, _, nearer, bugs = classify(verts, tris, rays[clear], got[clear], tb[clear], ref[clear],
                                   ref_tb[clear])
     assert bugs == [] and nearer == []
+
+
+# A ray from far away visits up to 10 times the nodes of one from near by; a
+# walk of the whole tree visits 1,000 times as many and more.
+SLOWER = 60
+
+
+def timed(verts, tris, rays):
+    """Seconds of the traversal alone (the build's are taken off) and results."""
+    best = []
+    for r in (rays, rays[:0]):
+        took = []
+        for _ in range(3):
+            t = time.perf_counter()
+            got = db.host_check_raycast(verts, tris, r)
+            took.append(time.perf_counter() - t)
+            if r is rays:
+                res = got
+        best.append(min(took))
+    return max(best[0] - best[1], 0.0), res
+
+
+@pytest.mark.parametrize("sizes", [100, 10000])
+def test_rays_from_far_away_do_not_visit_the_whole_tree(sizes):
+    """The margin is bounded by the nodes' own size."""
+    verts, tris = grid(200, 1.0, 0.6, np.random.default_rng(4))
+    verts, tris = verts.astype(np.float32), tris.astype(np.uint32)
+
+    def aimed(dist):
+        rng = np.random.default_rng(5)
+        rays = np.zeros((400, 8), np.float32)
+        p = verts[rng.integers(0, len(verts), 400)].astype(np.float64)
+        d = rng.normal(size=(400, 3))
+        d[:, 1] = np.abs(d[:, 1]) + 0.5
+        d /= np.linalg.norm(d, axis=1, keepdims=True)
+        o = (p + d * dist).astype(np.float32)
+        rays[:, 0:3] = o
+        rays[:, 4:7] = (p - o) / np.linalg.norm(p - o, axis=1, keepdims=True)
+        rays[:, 7] = np.inf
+        return rays
+
+    base, _ = timed(verts, tris, aimed(1.0))
+    took, _ = timed(verts, tris, aimed(float(sizes)))
+    assert took < SLOWER * base + 0.1, (took, base)
 
 
 @pytest.mark.gpu
