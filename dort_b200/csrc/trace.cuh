@@ -413,9 +413,17 @@ DG_HD void trav_init(TravState& s, const TraceScene& sc, float ox, float oy, flo
   s.near1 = s.ix < 0.f ? 0xaau : 0x55u;
   s.wt = wt_setup(dx, dy, dz);
   s.sp = 0;
-  // root group: one child with an empty internal-slot mask -> node 0; an
-  // empty tree starts finished
-  s.group = make_uint2(0u, sc.node_count ? 1u : 0u);
+  // root group: one child with an empty internal-slot mask -> node 0.  An empty
+  // tree or interval starts finished.  So does a ray that leaves its origin away
+  // from every box on some axis, from so far off that its distances overflow: the
+  // box test would subtract infinite distances and let every box pass.  A ray
+  // without a position on any axis (a NaN origin or direction) would pass every
+  // box too; the triangle test reports NaN distances as hits, and those of the
+  // last node (leaves only) do as well as any.
+  const float out = DG_MAX3(ox * s.ix, oy * s.iy, oz * s.iz);
+  const bool undefined = out != out;
+  const bool open = undefined ? t_min <= t_max : out <= 2e38f && !(t_max < t_min);
+  s.group = make_uint2(undefined ? sc.node_count - 1u : 0u, sc.node_count && open ? 1u : 0u);
 }
 
 // Traversal stacks.  A node group is pushed per level descended, so a ray's
@@ -566,7 +574,7 @@ DG_HD bool trav_tri(TravState& s, const TraceScene& sc, uint2& leaf) {
 // the closest hit, or for ANY_HIT the first hit found, or prim = kMiss).
 template<bool ANY_HIT, bool EXACT_MT, class Stack, int WT = kTriMt>
 DG_HD bool trav_step(TravState& s, const TraceScene& sc, Stack& stack) {
-  if(!group_left(s)) { return true; }   // an empty tree
+  if(!group_left(s)) { return true; }   // an empty tree or interval
   uint2 leaf = trav_node(s, sc, stack);
   while(!leaf_empty(leaf)) {
     if(trav_tri<ANY_HIT, EXACT_MT, WT>(s, sc, leaf) && ANY_HIT) { return true; }
