@@ -349,15 +349,8 @@ def run_reference(args):
     from oracle import pyoracle as po
     threads = os.cpu_count() or 1
     verts, tris = scenes.random_triangles(N_TRIS, seed=1)
-    if po.ref_available():
-        rb = po.RefBvh(verts, tris, "sah", threads=threads)
-        cast = lambda r: rb.raycast(r, threads=threads)
-        kind = "reference"
-    else:
-        ob = po.OracleBvh(verts, tris, "sah")
-        cast = lambda r: ob.raycast(r)
-        kind = "port"
-        threads = 1
+    rb = po.RefBvh(verts, tris, "sah", threads=threads)
+    cast = lambda r: rb.raycast(r, threads=threads)
     per_step = 1 << 20     # bounded sample of the 16M-ray workload per step
     coh_all = scenes.pinhole_rays(4096, 2048)
     dif = scenes.diffuse_rays(verts, tris, per_step // 2, cast, seed=2)
@@ -376,8 +369,8 @@ def run_reference(args):
         "ms_per_step": dt / args.steps * 1e3, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": WORKLOAD, "tris": N_TRIS, "rays_per_step": N_RAYS},
-        "cpu_baseline": {"value": mrays, "unit": "Mrays/s", "cores": threads, "kind": kind,
-                         **host_info(),
+        "cpu_baseline": {"value": mrays, "unit": "Mrays/s", "cores": threads,
+                         "kind": "reference", **host_info(),
                          "sample": f"{len(sample)} rays per step (1/16 of the workload: "
                                    "every 16th coherent ray + diffuse rays of a smaller "
                                    "second pass), closest hit"},
@@ -574,16 +567,28 @@ def _ref_worker_render(seed):
     return secs
 
 
-def ref_pt_pool(procs):
+def ref_pt_pool(procs, init=_ref_worker_init, initargs=()):
+    """Worker processes that hold the reference's scene.  An executor and not
+    a multiprocessing.Pool: a worker that fails to start breaks it (the next
+    step raises), where the Pool starts another one for ever."""
+    import concurrent.futures as cf
     import multiprocessing as mp
-    ctx = mp.get_context("spawn")
-    return ctx.Pool(procs, initializer=_ref_worker_init)
+    return cf.ProcessPoolExecutor(procs, mp_context=mp.get_context("spawn"), initializer=init,
+                                  initargs=initargs)
 
 
 def ref_pt_step(pool, procs, step):
     t0 = time.perf_counter()
-    pool.map(_ref_worker_render, [1000 * step + k for k in range(procs)])
+    list(pool.map(_ref_worker_render, [1000 * step + k for k in range(procs)]))
     return time.perf_counter() - t0
+
+
+def ref_missing():
+    """Why the reference cannot run here, or None."""
+    from oracle import pyoracle as po
+    return None if po.ref_available() else (
+        "the compiled reference (oracle/_ref/libdort_ref.so) is not here, nor the sources to "
+        "build it from")
 
 
 def pt_reference_work(sd, n=1 << 15):
@@ -818,18 +823,21 @@ def measure_pt(args, ctx):
         rays_per_frame = stages["rays"]
         if world == 1 and not args.no_cpu:
             n_node, n_tri, nwork = pt_reference_work(sd)
-            procs = ref_procs()
-            pool = ref_pt_pool(procs)
-            ref_pt_step(pool, procs, 0)                  # builds + warms the workers
-            secs = ref_pt_step(pool, procs, 1)
-            pool.close()
-            cpu_value = procs * REF_SAMPLE_W * REF_SAMPLE_H / secs
-            cpu = {"value": cpu_value, "unit": "samples/s", "cores": procs, "kind": "reference",
-                   **host_info(),
-                   "sample": f"{procs} single-threaded reference PathRenderer processes (one "
-                             f"per logical core), each one {REF_SAMPLE_W}x{REF_SAMPLE_H} frame "
-                             f"at 1 spp of the same scene and camera ({secs:.1f}s); GGX "
-                             "conductor timed as Phong"}
+            why = ref_missing()
+            if why:
+                log(f"no CPU baseline: {why}")
+            else:
+                procs = ref_procs()
+                with ref_pt_pool(procs) as pool:
+                    ref_pt_step(pool, procs, 0)          # builds + warms the workers
+                    secs = ref_pt_step(pool, procs, 1)
+                cpu_value = procs * REF_SAMPLE_W * REF_SAMPLE_H / secs
+                cpu = {"value": cpu_value, "unit": "samples/s", "cores": procs,
+                       "kind": "reference", **host_info(),
+                       "sample": f"{procs} single-threaded reference PathRenderer processes (one "
+                                 f"per logical core), each one {REF_SAMPLE_W}x{REF_SAMPLE_H} "
+                                 f"frame at 1 spp of the same scene and camera ({secs:.1f}s); "
+                                 "GGX conductor timed as Phong"}
             # dominant stage: the extend (closest-hit) stage, over the frame's
             # extension rays (counted by the staged run)
             ext_rays = stages["extend_rays"]
@@ -929,13 +937,12 @@ def scene_input_bytes(sd: dict) -> int:
 
 def run_reference_pt(args):
     procs = ref_procs()
-    pool = ref_pt_pool(procs)
-    for w in range(args.warmup):
-        ref_pt_step(pool, procs, w)
-    secs = 0.0
-    for k in range(args.steps):
-        secs += ref_pt_step(pool, procs, 100 + k)
-    pool.close()
+    with ref_pt_pool(procs) as pool:
+        for w in range(args.warmup):
+            ref_pt_step(pool, procs, w)
+        secs = 0.0
+        for k in range(args.steps):
+            secs += ref_pt_step(pool, procs, 100 + k)
     value = procs * REF_SAMPLE_W * REF_SAMPLE_H * args.steps / secs
     line = {
         "impl": "reference", "metric": "samples/s at 1080p equal-RMSE, wavefront vs plain GPU",
@@ -1274,15 +1281,18 @@ def main():
     if args.impl == "reference":
         if int(os.environ.get("RANK", "0")) != 0:
             return
-        if args.workload in ("raycast",):
-            run_reference(args)
-        elif args.workload == "pt1080p":
-            run_reference_pt(args)
+        if args.workload in ("batch", "adjoint"):
+            why = "the reference has no batched or adjoint renderer"
+        elif args.workload == "cornell":
+            why = "the reference arm times the pt1080p and raycast workloads only"
         else:
-            why = ("the reference has no batched or adjoint renderer"
-                   if args.workload in ("batch", "adjoint") else
-                   "the reference arm times the pt1080p and raycast workloads only")
+            why = ref_missing()
+        if why:
             print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+        elif args.workload == "raycast":
+            run_reference(args)
+        else:
+            run_reference_pt(args)
         return
     run_dort(args)
 
