@@ -820,7 +820,8 @@ def measure_pt(args, ctx):
         hbm, peak_kind = peaks()
         rl = None
         cpu = None
-        rays_per_frame = stages["rays"]
+        # the rays traced; the paths' rays of scenes with triangle lights are more
+        rays_per_frame = (stages["extend_rays"] + stages["shadow_rays"] + stages["neeb_rays"])
         if world == 1 and not args.no_cpu:
             n_node, n_tri, nwork = pt_reference_work(sd)
             why = ref_missing()
@@ -1047,7 +1048,7 @@ def measure_batch(args, ctx, steps, warmup, mega_warmup=True):
             "config": {"workload": BATCH_WORKLOAD, "jobs": len(jobs), "samples": samples,
                        "megakernel_samples_per_s": world * samples / (mega_ms / 1e3),
                        "batch_over_megakernel": (mega_ms / (ms / steps)),
-                       "rays_per_batch": st["rays"], "waves": st["waves"],
+                       "path_rays_per_batch": st["rays"], "waves": st["waves"],
                        "queue_capacity": tuning["queue_capacity"], "autotune": tuned,
                        "bvh_build": built, "bvh_build_ms_total": round(bvh_ms, 1),
                        "scene_create_s_total": round(create_s, 3)},

@@ -207,7 +207,8 @@ class Scene:
             ctypes.c_void_p(d_out), ctypes.c_void_p(stream)))
 
     def wavefront_stage_times(self, params: _abi.RenderParams, tuning: dict | None = None):
-        """Per-stage milliseconds of one frame run wave by wave (measurement)."""
+        """Per-stage milliseconds of one frame run wave by wave (measurement);
+        "rays" counts the paths' rays, the stages' rays those traced."""
         ms = (ctypes.c_double * 6)()
         rays = (ctypes.c_double * 4)()
         t = wavefront_tuning(**tuning) if tuning else None

@@ -710,8 +710,9 @@ __device__ __forceinline__ void wave_begin(WfDev& w) {
   *ctr_at(w.ctr, C_MORE) = more ? 1u : 0u;
 }
 
-// One thread of the wave's last kernel: the wave's rays are counted, the shade
-// queues consumed.  (Its own queues stay until the next wave_begin.)
+// One thread of the wave's last kernel: the rays of the wave's paths are counted
+// (those past their light too, as the megakernel counts them), the shade queues
+// consumed.  (Its own queues stay until the next wave_begin.)
 __device__ __forceinline__ void wave_end(WfDev& w) {
   const uint32_t wave = wave_of(w);
   unsigned long long* rays = reinterpret_cast<unsigned long long*>(ctr_at(w.ctr, C_RAYS_LO));
@@ -1743,9 +1744,9 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
   SingleJob<G> jobs{s->pt, pp};
   WfGrids g = wf_grids<SingleJob<G>>(tn);
   wf->dev.sorted = tn.sort;
-  // more[0]: loop flag; more[1..]: the counters C_ACT0 .. C_NB_PAST of the wave
+  // more[0]: loop flag; more[1..]: the counters C_ACT0 .. C_NEEB of the wave
   uint32_t* more = nullptr;
-  DG_CUDA(host_pinned_alloc(&more, 16 * sizeof(uint32_t)));
+  DG_CUDA(host_pinned_alloc(&more, 8 * sizeof(uint32_t)));
   cudaEvent_t ev[6];
   for(auto& e : ev) { cudaEventCreate(&e); }
   for(int k = 0; k < 6; ++k) { ms[k] = 0.0; }
@@ -1766,7 +1767,7 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
     wf_launch_light<SingleJob<G>>(jobs, wf->dev, tn, g, LIGHT_NEEB | LIGHT_END, st);
     cudaEventRecord(ev[5], st);
     cudaMemcpy2DAsync(more + 1, sizeof(uint32_t), wf->dev.ctr, kCtrStride * sizeof(uint32_t),
-                      sizeof(uint32_t), C_NB_PAST + 1, cudaMemcpyDeviceToHost, st);
+                      sizeof(uint32_t), C_NEEB + 1, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(more, ctr_at(wf->dev.ctr, C_MORE), sizeof(uint32_t), cudaMemcpyDeviceToHost,
                     st);
     ok = cudaStreamSynchronize(st) == cudaSuccess;
@@ -1778,7 +1779,7 @@ static int stage_times_g(dort_scene* s, const PtParams& pp, const WfTuning& tn, 
     if(ok) {
       stage_rays[0] += double(more[1 + C_ACT0 + (wave & 1u)]);
       stage_rays[1] += double(more[1 + C_SHADOW]);
-      stage_rays[2] += double(more[1 + C_NEEB]) + double(more[1 + C_NB_PAST]);
+      stage_rays[2] += double(more[1 + C_NEEB]);
     }
     if(!*more) { break; }
   }

@@ -33,7 +33,7 @@ void wavefront_destroy(Wavefront* wf);
 int wavefront_render(dort_scene* s, const PtParams& pp, const WfTuning& tn, float* d_out,
                      cudaStream_t st);
 // ms: per-stage milliseconds (5) and waves; stage_rays: extend, shadow and
-// BSDF-strategy rays of the frame.
+// BSDF-strategy rays that the frame traced.
 int wavefront_stage_times(dort_scene* s, const PtParams& pp, const WfTuning& tn,
                           float* d_out, cudaStream_t st, double ms[6], double stage_rays[3]);
 struct WavefrontBatch;

@@ -427,8 +427,12 @@ typedef struct dort_wavefront_tuning {
                                   MIS BSDF strategy, or sample_all_lights) */
 } dort_wavefront_tuning;
 
-/* out_stats (optional, 4 doubles): rays traced, samples kept, kernel
- * milliseconds, waves.  tuning may be NULL (automatic). */
+/* out_stats (optional, 4 doubles): rays of the paths, samples kept, kernel
+ * milliseconds, waves.  The rays are those that dort_gpu_render traces; the
+ * wavefront decides some of them without a traversal (a BSDF-strategy ray
+ * towards a triangle light that passes the triangle by contributes nothing
+ * whatever it hits), see dort_gpu_wavefront_stage_times for the ones traced.
+ * tuning may be NULL (automatic). */
 int dort_gpu_render_wavefront(dort_scene* scene, const dort_render_params* params,
                               const dort_wavefront_tuning* tuning, float* out_rgb,
                               double* out_stats);
@@ -459,8 +463,8 @@ int dort_gpu_batch_render(dort_batch* batch, void* stream);
 int dort_gpu_batch_image(dort_batch* batch, uint32_t job, float* out_rgb);
 /* Device pointer of job `job`'s image inside the batch. */
 int dort_gpu_batch_image_device(dort_batch* batch, uint32_t job, const float** out_d_rgb);
-/* out[0] = rays traced, out[1] = waves, out[2] = 1 if the wave bound was hit,
- * out[3] = total samples (waits for the last render). */
+/* out[0] = rays of the paths (as dort_gpu_render_wavefront counts them), out[1]
+ * = waves, out[2] = 1 if the wave bound was hit, out[3] = total samples (waits for the last render). */
 int dort_gpu_batch_stats(dort_batch* batch, double out[4]);
 int dort_gpu_batch_destroy(dort_batch* batch);
 
@@ -488,9 +492,10 @@ int dort_gpu_autotune_batch(const dort_batch_job* jobs, uint32_t job_count, doub
 /* Measurement entry: renders the same frame wave by wave from the host
  * (without the graph) with CUDA events around each stage; out_ms[0..4] =
  * total milliseconds of regen, extend, shade, shadow, neeb; out_ms[5] = waves;
- * out_rays (optional, 4 doubles) = rays traced in total, by the extend stage
- * (closest hit), by the shadow stage (any hit) and by the BSDF-strategy stage
- * (closest hit). */
+ * out_rays (optional, 4 doubles) = rays of the paths in total (as
+ * dort_gpu_render_wavefront counts them), and the rays traced by the extend
+ * stage (closest hit), by the shadow stage (any hit) and by the BSDF-strategy
+ * stage (closest hit).  The three add up to the rays traced. */
 int dort_gpu_wavefront_stage_times(dort_scene* scene, const dort_render_params* params,
                                    const dort_wavefront_tuning* tuning, double out_ms[6],
                                    double out_rays[4]);
@@ -522,7 +527,8 @@ int dort_gpu_wavefront_stage_times(dort_scene* scene, const dort_render_params* 
 /* The scene's last backward pass (4 doubles): engine (0: wavefront, 1:
  * megakernel, 2: wavefront whose overflowing samples outnumbered its list,
  * then the megakernel), samples traced a second time because their terms
- * overflowed the wavefront's per-path log, wavefront rays, waves. */
+ * overflowed the wavefront's per-path log, rays of the wavefront's paths,
+ * waves. */
 int dort_gpu_adjoint_stats(dort_scene* scene, double* out_stats);
 
 /* Testing aid: the list of samples a wavefront backward pass traces a second
