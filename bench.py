@@ -912,7 +912,8 @@ def measure_pt(args, ctx):
                     "scene_create_ms": round(scene_create_ms, 1),
                     "scene_h2d_bytes": scene_input_bytes(sd),
                     "scene_device_bytes": int(st["device_bytes"])},
-            "gpu_launches": args.steps * int(stages["waves"] * 6 + 2),
+            # four kernels a wave, one before the first and one after the last
+            "gpu_launches": args.steps * int(stages["waves"] * 4 + 2),
             "clocks": clk,
         }
     sc.close()
@@ -1053,7 +1054,7 @@ def measure_batch(args, ctx, steps, warmup, mega_warmup=True):
                        "bvh_build": built, "bvh_build_ms_total": round(bvh_ms, 1),
                        "scene_create_s_total": round(create_s, 3)},
             "roofline": None, "cpu_baseline": None,
-            "e2e": None, "gpu_launches": steps * int(st["waves"] * 6 + 2), "clocks": clk,
+            "e2e": None, "gpu_launches": steps * int(st["waves"] * 4 + 2), "clocks": clk,
         }
     b.close()
     for sc, _ in jobs:
