@@ -339,7 +339,11 @@ extern "C" int dort_gpu_adjoint_backward(dort_scene* scene, const dort_render_pa
   // on 200k triangles took 13 waves and 9.8 ms with one for every four samples.
   const uint64_t units = uint64_t((pp.width + 7) / 8) * ((pp.height + 3) / 4) * 32 *
                          ((uint64_t(pp.spp) + kWfUnitSamples - 1) / kWfUnitSamples);
-  const uint32_t capacity = uint32_t((std::min<uint64_t>(units, kAdjSlots) + 31) & ~uint64_t(31));
+  auto slots = [](uint64_t n) {
+    return uint32_t((std::min<uint64_t>(n, kAdjSlots) + 31) & ~uint64_t(31));
+  };
+  uint32_t capacity = slots(units);
+  if(scene->adjoint_slots_fit) { capacity = std::min(capacity, scene->adjoint_slots_fit); }
   // samples whose terms overflow the wavefront's log, traced again: a list
   // of up to every sample of the frame, at most 2^24
   uint32_t overflow_cap = uint32_t(std::min<uint64_t>(uint64_t(npix) * pp.spp, kAdjListMax));
@@ -407,14 +411,22 @@ extern "C" int dort_gpu_adjoint_backward(dort_scene* scene, const dort_render_pa
   } else if(ok) {
     ok = cudaMemsetAsync(d_list_n, 0, sizeof(uint32_t), st) == cudaSuccess;
     WfTuning tn{};
-    tn.capacity = capacity;
     tn.trace_block = 128;
     tn.shade_block = 128;
-    if(ok) {
+    // where the queues and the term log do not fit the device memory, fewer
+    // slots do, down to one for every four units (836 bytes a slot); what fits is
+    // remembered, so that later steps do not try the larger ones again
+    const uint32_t fewest = std::min(capacity, slots((units + 3) / 4));
+    for(rc = DORT_OK; ok;) {
+      tn.capacity = capacity;
       rc = wavefront_adjoint(scene, pp, tn, d_img, d_ga, d_ge, d_list, overflow_cap, d_list_n,
                              st);
-      if(rc != DORT_OK) { return rc; }
+      if(rc != DORT_ERR_OOM || capacity <= fewest) { break; }
+      clear_error();
+      capacity = std::max(fewest, (capacity / 2) & ~31u);
+      scene->adjoint_slots_fit = capacity;
     }
+    if(rc != DORT_OK) { return rc; }
     uint32_t listed = 0;
     ok = ok && cudaMemcpyAsync(&listed, d_list_n, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                st) == cudaSuccess;

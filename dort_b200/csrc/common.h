@@ -114,6 +114,7 @@ struct dort_scene {
   // the adjoint's image gradient and triangle gradients (grow-only)
   void* d_adjoint = nullptr;
   size_t adjoint_bytes = 0;
+  uint32_t adjoint_slots_fit = 0;       // path slots that its queues had memory for (0: no limit met)
   // the last backward pass: engine (0 wavefront, 1 megakernel, 2 wavefront
   // then megakernel), samples traced a second time, rays, waves
   double adjoint_stats[4] = {0.0, 0.0, 0.0, 0.0};
