@@ -89,7 +89,7 @@ N_RAYS = 16 * 1024 * 1024
 # workload, from the ncu capture summarised in
 # profiles/raycast_kernel_1Mtri_16Mrays.md (dram__bytes_read.sum +
 # dram__bytes_write.sum); reported as the roofline's traffic.
-RAYCAST_TRAFFIC_BYTES = 815.3e6
+RAYCAST_TRAFFIC_BYTES = 814.2e6
 # The bound that applies to the ray cast beside the HBM roofline (whose
 # algorithmic bytes count the reference's binary-tree work, more than the
 # wide tree does, so its frac exceeds 1): issue slots.  Figures of one
@@ -98,9 +98,9 @@ RAYCAST_LIMITER = {
     "bound": "issue slots (divergent traversal)",
     "source": "ncu capture of one raycast_kernel launch, "
               "profiles/raycast_kernel_1Mtri_16Mrays.md",
-    "issue_slots_busy": 0.757, "simt_efficiency": 23.6 / 32, "achieved_occupancy": 0.495,
-    "l1_data_pipe": 0.669, "dram_throughput": 0.023,
-    "top_stall": "long_scoreboard, 3.04 cycles per issue",
+    "issue_slots_busy": 0.760, "simt_efficiency": 23.5 / 32, "achieved_occupancy": 0.495,
+    "l1_data_pipe": 0.650, "dram_throughput": 0.023,
+    "top_stall": "long_scoreboard, 2.90 cycles per issue",
 }
 WORKLOAD = "raycast: 1M random tris (SAH BVH), 16M rays (8M coherent pinhole 4096x2048 + 8M diffuse bounce), closest hit"
 
@@ -532,9 +532,9 @@ PT_WORKLOAD = ("pt1080p: wavefront path tracing 1920x1080, 256 spp, max depth 16
 REF_SAMPLE_W, REF_SAMPLE_H = 480, 270
 # DRAM bytes (read + write) of one wf_extend launch over a full queue
 # (4,194,304 rays, a wave of the 16-spp frame), from
-# the ncu capture summarised in profiles/wf_extend_pt1080p.md: 613 MB, 146 B
+# the ncu capture summarised in profiles/wf_extend_pt1080p.md: 599 MB, 143 B
 # per ray; reported as the roofline's traffic.
-EXTEND_TRAFFIC_BYTES = 612.6e6
+EXTEND_TRAFFIC_BYTES = 599.0e6
 EXTEND_TRAFFIC_RAYS = 4194304
 # The bound that applies to the extension stage beside the HBM roofline:
 # issue slots and latency.  Figures of one wf_extend launch under
@@ -545,10 +545,10 @@ EXTEND_LIMITER = {
     "bound": "issue slots and node-fetch latency (divergent traversal)",
     "source": "ncu capture of one full-queue wf_extend launch, "
               "profiles/wf_extend_pt1080p.md",
-    "issue_slots_busy": 0.655, "simt_efficiency": 24.23 / 32, "achieved_occupancy": 0.470,
-    "occupancy_limit": 0.5, "l1_data_pipe": 0.539, "l2_throughput": 0.196,
-    "dram_throughput": 0.095,
-    "top_stall": "long_scoreboard (L1/L2 node and stack loads), 5.25 cycles per issue",
+    "issue_slots_busy": 0.666, "simt_efficiency": 24.16 / 32, "achieved_occupancy": 0.469,
+    "occupancy_limit": 0.5, "l1_data_pipe": 0.526, "l2_throughput": 0.194,
+    "dram_throughput": 0.093,
+    "top_stall": "long_scoreboard (L1/L2 node and stack loads), 5.04 cycles per issue",
 }
 
 _ref_worker_scene = None

@@ -2,8 +2,8 @@
 // Plain host C++ (no CUDA types), so the rules can be checked on a machine
 // without a GPU.
 //
-// A path slot holds about 184 bytes of path state, queues and sort buffers,
-// plus 156 bytes of direct-lighting queues per light a vertex samples
+// A path slot holds 168 bytes of path state, queues and sort buffers (counted
+// as 184, so that the allocation's padding is on the safe side), plus 156 bytes of direct-lighting queues per light a vertex samples
 // (nee_mult: the light count when every light is sampled, else 1): two
 // shadow entries (slot index, origin, direction, contribution) and one
 // BSDF-strategy entry per light, wavefront.cu (wf_alloc).  The queues'

@@ -50,11 +50,11 @@ struct RaycastQueue {
 
 // 64 registers (8 resident blocks): 9 and 10 blocks measured 2 and 9 % slower
 // on incoherent rays (spills), 6 and 7 no faster.  What bounds it on the
-// 1M-triangle soup (4M rays): camera rays (1.45 ms), instruction issue (74 % of
-// the active cycles, 24.4 threads an instruction); bounce rays (2.21 ms), the
+// 1M-triangle soup (4M rays): camera rays (1.50 ms), instruction issue (74 % of
+// the active cycles, 24.4 threads an instruction); bounce rays (2.24 ms), the
 // L1 data pipe (82 %) and issue (69 %, 22.9 threads) together.  The same rays
 // one per lane to its end took the pipe to 82 % with 13.4 threads an
-// instruction; 16.8M rays, half of each: 12.0 ms then, 7.2 ms now.
+// instruction; 16.8M rays, half of each: 12.0 ms then, 7.3 ms now.
 template<bool ANY_HIT, int WT = kTriMt>
 __global__ void __launch_bounds__(kRaycastBlock, 8)
 raycast_kernel(TraceScene sc, const float4* __restrict__ rays, uint32_t ray_count,

@@ -17,8 +17,8 @@
 // Measured on the 1M-triangle soup: a warp's 32 diffuse bounce rays took 59
 // node steps with 16.5 lanes active and 115 triangle tests with 3.5 lanes
 // active one ray per lane to the end; 37.5 steps with 26 lanes and 34 tests
-// with 12 lanes this way (4M such rays: 3.61 ms against 2.47 ms; the camera
-// rays of the same scene 1.69 against 1.65 ms).
+// with 12 lanes this way (4M such rays: 3.61 ms against 2.47 ms when it came, 2.24
+// now; the camera rays of the same scene 1.69 against 1.65, now 1.50 ms).
 #pragma once
 #include "trace.cuh"
 
